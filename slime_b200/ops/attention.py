@@ -91,6 +91,12 @@ def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, 
     return out, lse
 
 
+def _key_parts(ctas: int, group: int, sms: int) -> int:
+    """CTAs that share the query heads of one (key tile, kv head) in the backward: enough to give every SM about three, so that the
+    long tiles of one SM find company on the others; the parts are summed in fp32 afterwards."""
+    return max(1, min(group, -(-3 * sms // max(ctas, 1))))
+
+
 def flash_bwd(q, k, v, o, d_o, lse, seg, scale, dq=None, dk=None, dv=None):
     """Backward kernel launches (delta, dK/dV pass, dQ pass). Gradient tensors may be views into one packed buffer.
     Rows outside every segment are zeroed here when the outputs are allocated here, else left to the caller."""
@@ -104,9 +110,12 @@ def flash_bwd(q, k, v, o, d_o, lse, seg, scale, dq=None, dk=None, dv=None):
     dv = torch.zeros(Tk, Hkv, D, dtype=v.dtype, device=v.device) if dv is None else dv
     delta = torch.empty_like(lse)
     nseg = seg.shape[0]
-    fn = _lib.bind("sb_flash_bwd", [_lib.P] * 11 + [_lib.I] * 17 + [_lib.F, _lib.P, _lib.P])
+    k_tiles = -(-Tk // 128) + nseg
+    parts = _key_parts(k_tiles * Hkv, Hq // Hkv, _lib.sm_count(q.device))
+    partial = torch.empty(parts, 2, Tk, Hkv * D, dtype=torch.float32, device=q.device) if parts > 1 else None
+    fn = _lib.bind("sb_flash_bwd", [_lib.P] * 11 + [_lib.I, _lib.P] + [_lib.I] * 17 + [_lib.F, _lib.P, _lib.P])
     rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), seg.data_ptr(), nseg, -(-Tq // 128) + nseg, -(-Tk // 128) + nseg, Tq, Tk,
+            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.ptr(partial), parts, seg.data_ptr(), nseg, -(-Tq // 128) + nseg, k_tiles, Tq, Tk,
             Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dq.stride(0), dk.stride(0),
             dv.stride(0), lse.stride(0), float(scale), _lib.ptr(_lib.status_word(q.device)), _lib.stream())  # fmt: skip
     _lib.check(rc, "sb_flash_bwd")

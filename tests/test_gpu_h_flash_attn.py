@@ -123,3 +123,41 @@ def test_rope_attention_node_matches_reference(kernels):
     want = run("cpu", torch.float32)
     for name, g, r in zip(("out", "dqkv", "dq_norm_w", "dk_norm_w"), got, want):
         _close(g, r, name, 4e-2 * float(r.abs().max()) + 1e-3, 4e-2)
+
+
+@pytest.mark.parametrize("lens,Hq,Hkv,D", [
+    ([1 + 37 * i % 191 for i in range(70)], 14, 2, 64),  # more segments than one step of the table's search, query heads of a key tile split 7 ways
+    ([63, 64, 65, 191, 192, 193], 6, 2, 128),  # edges of the streamed blocks, parts of one and two heads
+    ([7201], 16, 8, 64),  # enough key tiles for the machine: one CTA for all heads of a group
+])  # fmt: skip
+def test_flash_backward_splits_and_tables(kernels, lens, Hq, Hkv, D):
+    """The launch shapes of the backward: every split of a group's query heads gives the same sums, and long tables are searched right.
+    Bounds: P and dS are rounded to bf16 (2^-9 each) and the outputs once more, on sums whose terms have random signs."""
+    from slime_b200.ops import _lib, attention
+
+    torch.manual_seed(len(lens))
+    T = sum(lens)
+    q, d_o = ((torch.randn(T, Hq, D, device="cuda") * 0.8).to(torch.bfloat16) for _ in range(2))
+    k, v = ((torch.randn(T, Hkv, D, device="cuda") * 0.8).to(torch.bfloat16) for _ in range(2))
+    seg = attention.segments_from_cu_seqlens(torch.tensor([0] + lens, device="cuda").cumsum(0))
+    out, lse = attention.flash_fwd(q, k, v, seg, D**-0.5)
+    got = attention.flash_bwd(q, k, v, out, d_o, lse, seg, D**-0.5)
+    again = attention.flash_bwd(q, k, v, out, d_o, lse, seg, D**-0.5)
+    _lib.check_status("cuda")
+    at, want = 0, [torch.zeros_like(x, dtype=torch.float32) for x in (q, k, v)]
+    for n in lens:
+        for h in range(Hkv):
+            g = slice(h * Hq // Hkv, (h + 1) * Hq // Hkv)
+            qs, ks, vs, ds = q[at : at + n, g].double(), k[at : at + n, h].double(), v[at : at + n, h].double(), d_o[at : at + n, g].double()
+            p = torch.einsum("igd,jd->gij", qs, ks) * D**-0.5
+            p = p.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), -math.inf).softmax(-1)
+            dp = torch.einsum("igd,jd->gij", ds, vs)
+            s = p * (dp - (p * dp).sum(-1, keepdim=True)) * D**-0.5
+            want[0][at : at + n, g] = torch.einsum("gij,jd->igd", s, ks).float()
+            want[1][at : at + n, h] = torch.einsum("gij,igd->jd", s, qs).float()
+            want[2][at : at + n, h] = torch.einsum("gij,igd->jd", p, ds).float()
+        at += n
+    for name, a, b, w in zip(("dq", "dk", "dv"), got, again, want):
+        assert torch.equal(a, b), f"{name} is not the same twice"
+        rel = float((a.float() - w).norm() / w.norm())
+        assert rel < 3 * 2**-8, f"{name}: {rel}"
