@@ -9,14 +9,20 @@
 // k_len > q_len, and a context-parallel rank passes its local query chunk against a prefix of the gathered keys.
 // GQA: query head h uses kv head h / (Hq / Hkv).
 //
-// One CTA = one 128-row query tile of one head. 6 warps: warp 0 issues TMA loads (Q once, K / V tiles of 128 keys
-// through a 2-stage ring), warp 1 owns TMEM and issues tcgen05.mma, warps 2-5 are the softmax: thread r owns query row
-// r (= TMEM lane r).
+// One CTA = 256 query rows of one head, as two tiles of 128. 10 warps: warp 0 issues TMA loads (Q once, K / V tiles of 128 keys
+// through a 2-stage ring that both tiles read), warp 1 owns TMEM and issues tcgen05.mma, and each query tile g has a softmax group of
+// four warps: thread r owns query row r (= TMEM lane r).
 //
-//   S_j  = Q K_j^T            M 128, N 128, K D        TMEM, two buffers: S_{j+1} is issued before the softmax of tile j
-//   P_j  = 2^(S_j*c - m)      registers -> bf16 -> shared memory (128B-swizzled, the A operand of the next product)
-//   O   += P_j V_j            M 128, N D,  K 128       accumulated in TMEM over all tiles of the row
+//   S_g  = Q_g K_j^T          M 128, N 128, K D        TMEM
+//   P_g  = 2^(S_g*c - m)      TMEM -> registers -> bf16 over the scores it came from (the A operand of the next product)
+//   O_g += P_g V_j            M 128, N D,  K 128       accumulated in TMEM over all tiles of the row
 //
+// What bounds it: the chain scores -> softmax -> product of a tile. With one tile per CTA the tensor cores stood still during the
+// softmax and the softmax during the products; with two, group 0's softmax runs beside the products of tile 1 and the other way
+// round, K and V are read from L2 half as often, and P does not pass through shared memory. Measured, before -> after:
+// 8011 + 1187 tokens, 32 / 8 heads of 128: 901 -> 520 us (1034 TFLOP/s); 19 sequences of 384 to 1284 tokens, 14 / 2 heads of 64:
+// 167 -> 101 us; 4096 tokens, 32 / 8 heads of 128: 267 -> 154 us.
+// CTAs are ordered heads first and last query rows (most keys) first.
 // The running maximum m is only raised when a tile exceeds it by more than 2^8 (decided per warp): otherwise the stale
 // maximum keeps being used, p stays below 256 and O needs no correction; when it is raised the owning thread rescales
 // its O row in TMEM (tcgen05.ld / st) before the next product is issued. Scores live in the log2 domain.
@@ -26,20 +32,19 @@
 
 namespace sb {
 
-constexpr int FA_BM = 128;       // query rows per CTA
+constexpr int FA_BM = 128;       // query rows of one tile; a CTA has two
 constexpr int FA_BN = 128;       // keys per tile
-constexpr int FA_THREADS = 192;  // TMA warp, MMA warp, 4 softmax warps
+constexpr int FA_THREADS = 320;  // TMA warp, MMA warp, 2 x 4 softmax warps
 constexpr int FA_KV_STAGES = 2;
 
 template <int D>
 struct FaSmem {
   static constexpr int NCH = D / 64;                  // 128-byte chunks of the head dim
-  static constexpr int Q_BYTES = FA_BM * 128 * NCH;   // [NCH][128 rows][128 B]
+  static constexpr int Q_BYTES = FA_BM * 128 * NCH;   // one query tile, [NCH][128 rows][128 B]; its output is staged here at the end
   static constexpr int KV_BYTES = FA_BN * 128 * NCH;  // one K or V tile
-  static constexpr int P_BYTES = FA_BM * FA_BN * 2;   // [2 chunks of 64 keys][128 rows][128 B]
   static constexpr int BAR_BYTES = 256;
-  static constexpr int TOTAL = Q_BYTES + 2 * FA_KV_STAGES * KV_BYTES + P_BYTES + BAR_BYTES + 1024;  // +1024: alignment
-  static constexpr int TMEM_COLS = 512;  // S0 @0, S1 @128, O @256 (D columns)
+  static constexpr int TOTAL = 2 * Q_BYTES + 2 * FA_KV_STAGES * KV_BYTES + BAR_BYTES + 1024;  // +1024: alignment
+  static constexpr int TMEM_COLS = 512;  // S_0 @0, S_1 @128 (P_g over the first 64 columns of S_g), O_0 @256, O_1 @256 + D
 };
 
 __device__ __forceinline__ float fa_exp2(float x) {
@@ -56,30 +61,29 @@ template <int D>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
-                 const int* __restrict__ seg, int nseg, int Hq, int Hkv, int out_stride, int lse_stride, float scale,
+                 const int* __restrict__ seg, int nseg, int Hq, int Hkv, int tiles, int out_stride, int lse_stride, float scale,
                  int* status) {
   using S = FaSmem<D>;
   constexpr int NCH = S::NCH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + S::Q_BYTES;
+  uint8_t* sQ = smem;                                  // [2 tiles]
+  uint8_t* sK = sQ + 2 * S::Q_BYTES;
   uint8_t* sV = sK + FA_KV_STAGES * S::KV_BYTES;
-  uint8_t* sP = sV + FA_KV_STAGES * S::KV_BYTES;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(sP + S::P_BYTES);
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sV + FA_KV_STAGES * S::KV_BYTES);
   uint64_t* k_full = q_full + 1;
   uint64_t* k_empty = k_full + FA_KV_STAGES;
   uint64_t* v_full = k_empty + FA_KV_STAGES;
   uint64_t* v_empty = v_full + FA_KV_STAGES;
-  uint64_t* s_full = v_empty + FA_KV_STAGES;  // [2]
-  uint64_t* p_full = s_full + 2;
-  uint64_t* o_done = p_full + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  uint64_t* s_full = v_empty + FA_KV_STAGES;  // [2 groups] scores of a tile are in TMEM, and every earlier product has finished
+  uint64_t* p_full = s_full + 2;              // [2 groups] P is in TMEM (4 arrivals)
+  uint64_t* o_full = p_full + 2;              // [2 groups] the group's last product has finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* work = reinterpret_cast<int*>(tmem_slot + 2);  // [0] segment or -1, [1] tile in segment
+  int* work = reinterpret_cast<int*>(tmem_slot + 2);  // [0] segment or -1, [1] pair of tiles in the segment
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y;
+  const int h = blockIdx.x % Hq;
   const int kvh = h / (Hq / Hkv);
 
   if (threadIdx.x == 0) {
@@ -90,10 +94,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
     }
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 4);  // one arrival per softmax warp
-    mbar_init(o_done, 1);
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(&s_full[g], 1);
+      mbar_init(&p_full[g], 4);  // one arrival per softmax warp of the group
+      mbar_init(&o_full[g], 1);
+    }
     *cta_abort = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
@@ -106,20 +111,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   pdl_wait();
   pdl_launch_dependents();
-  if (threadIdx.x == 0) {
-    // which (segment, tile) is this CTA's? Tiles are numbered segment by segment.
-    int t = blockIdx.x, found = -1, tile = 0;
-    for (int s = 0; s < nseg; ++s) {
-      const int nt = (seg[4 * s + 1] + FA_BM - 1) / FA_BM;
-      if (t < nt) {
-        found = s;
-        tile = t;
-        break;
-      }
-      t -= nt;
+  if (warp == 0) {
+    int pair;
+    const int found = segment_of_tile(seg, nseg, 1, 2 * FA_BM, tiles - 1 - static_cast<int>(blockIdx.x / Hq), pair);
+    if (lane == 0) {
+      work[0] = found;
+      work[1] = pair;
     }
-    work[0] = found;
-    work[1] = tile;
   }
   tc_fence_before();
   __syncthreads();
@@ -128,17 +126,25 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int sidx = work[0];
   if (sidx >= 0) {
     const int q_off = seg[4 * sidx], q_len = seg[4 * sidx + 1], k_off = seg[4 * sidx + 2], k_len = seg[4 * sidx + 3];
-    const int q0 = work[1] * FA_BM;              // first query row of this tile inside the segment
+    const int q0 = work[1] * 2 * FA_BM;          // first query row of this CTA inside the segment
     const int shift = k_len - q_len;             // query i sees keys j <= shift + i
-    const int kv_hi = min(k_len, shift + q0 + FA_BM);
-    const int n_kv = (kv_hi + FA_BN - 1) / FA_BN;
+    // key tiles of the two query tiles (none for a second tile that lies past the segment)
+    auto key_tiles = [&](int g) {
+      const int r0 = q0 + g * FA_BM;
+      return r0 < q_len ? (max(min(k_len, shift + r0 + FA_BM), 0) + FA_BN - 1) / FA_BN : 0;
+    };
+    const int n_of[2] = {key_tiles(0), key_tiles(1)};
+    const int n_kv = max(n_of[0], n_of[1]);
 
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
-        mbar_arrive_expect_tx(q_full, S::Q_BYTES);
+      if (lane == 0 && n_kv > 0) {
+        mbar_arrive_expect_tx(q_full, 2 * S::Q_BYTES);
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) tma_load_2d(sQ + c * (FA_BM * 128), &tmQ, q_full, h * D + c * 64, q_off + q0);
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+          for (int c = 0; c < NCH; ++c)
+            tma_load_2d(sQ + g * S::Q_BYTES + c * (FA_BM * 128), &tmQ, q_full, h * D + c * 64, q_off + q0 + g * FA_BM);
         for (int j = 0; j < n_kv; ++j) {
           const int st = j % FA_KV_STAGES;
           const uint32_t par = (j / FA_KV_STAGES) & 1;
@@ -156,170 +162,171 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
+      if (lane == 0 && n_kv > 0) {
         constexpr uint32_t idesc_s = make_idesc(FA_BM, FA_BN, 1, 1, 0, 0);
-        constexpr uint32_t idesc_o = make_idesc(FA_BM, D, 1, 1, 0, 1);  // B = V read MN-major
-        const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
-        auto issue_s = [&](int j) {
-          const uint32_t k_addr = smem_u32(sK + (j % FA_KV_STAGES) * S::KV_BYTES);
+        constexpr uint32_t idesc_o = make_idesc(FA_BM, D, 1, 1, 0, 1);  // A = P in TMEM, B = V read MN-major
+        auto issue_s = [&](int g, int j) {
+          const uint32_t q_addr = smem_u32(sQ + g * S::Q_BYTES), k_addr = smem_u32(sK + (j % FA_KV_STAGES) * S::KV_BYTES);
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
             const uint32_t off = (k >> 2) * (FA_BM * 128) + (k & 3) * 32;
-            umma_f16(tmem_base + (j & 1) * FA_BN, make_smem_desc(q_addr + off, 16, 1024, UMMA_SWIZZLE_128B),
+            umma_f16(tmem_base + g * FA_BN, make_smem_desc(q_addr + off, 16, 1024, UMMA_SWIZZLE_128B),
                      make_smem_desc(k_addr + off, 16, 1024, UMMA_SWIZZLE_128B), idesc_s, k != 0 ? 1u : 0u);
           }
-          umma_commit(&k_empty[j % FA_KV_STAGES]);
-          umma_commit(&s_full[j & 1]);
+          umma_commit(&s_full[g]);
         };
         bool ok = mbar_wait(q_full, 0, cta_abort, status, ERR_WAIT_FULL) &&
                   mbar_wait(&k_full[0], 0, cta_abort, status, ERR_WAIT_FULL);
         if (ok) {
           tc_fence_after();
-          issue_s(0);
+          for (int g = 0; g < 2; ++g)
+            if (n_of[g] > 0) issue_s(g, 0);
+          umma_commit(&k_empty[0]);
         }
         for (int j = 0; j < n_kv && ok; ++j) {
-          if (j + 1 < n_kv) {
-            // S_{j+1} goes to the other buffer (the softmax of tile j-1 has released it: its p_full was seen below)
-            ok = mbar_wait(&k_full[(j + 1) % FA_KV_STAGES], ((j + 1) / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+          ok = mbar_wait(&v_full[j % FA_KV_STAGES], (j / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+          const uint32_t v_addr = smem_u32(sV + (j % FA_KV_STAGES) * S::KV_BYTES);
+          for (int g = 0; g < 2 && ok; ++g) {
+            if (j >= n_of[g]) continue;
+            ok = mbar_wait(&p_full[g], j & 1, cta_abort, status, ERR_WAIT_TMEM_EMPTY);
             if (!ok) break;
             tc_fence_after();
-            issue_s(j + 1);
-          }
-          ok = mbar_wait(p_full, j & 1, cta_abort, status, ERR_WAIT_TMEM_EMPTY) &&
-               mbar_wait(&v_full[j % FA_KV_STAGES], (j / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t v_addr = smem_u32(sV + (j % FA_KV_STAGES) * S::KV_BYTES);
 #pragma unroll
-          for (int k = 0; k < FA_BN / 16; ++k) {
-            // A = P: K-major, 64-key chunks 16 KB apart; B = V tile [128 keys, D]: MN-major, 16 keys = 2048 B,
-            // 64-wide chunks of the head dim FA_BN * 128 B apart
-            const uint64_t da = make_smem_desc(p_addr + (k >> 2) * (FA_BM * 128) + (k & 3) * 32, 16, 1024, UMMA_SWIZZLE_128B);
-            const uint64_t db = make_smem_desc(v_addr + k * 2048, FA_BN * 128, 1024, UMMA_SWIZZLE_128B);
-            umma_f16(tmem_base + 2 * FA_BN, da, db, idesc_o, (j != 0 || k != 0) ? 1u : 0u);
+            for (int k = 0; k < FA_BN / 16; ++k) {
+              // A: 16 keys = 8 TMEM columns; B = V tile [128 keys, D]: MN-major, 16 keys = 2048 B, 64-wide chunks of the head dim
+              // FA_BN * 128 B apart
+              umma_f16_ts(tmem_base + 2 * FA_BN + g * D, tmem_base + g * FA_BN + k * 8,
+                          make_smem_desc(v_addr + k * 2048, FA_BN * 128, 1024, UMMA_SWIZZLE_128B), idesc_o, (j != 0 || k != 0) ? 1u : 0u);
+            }
+            if (j + 1 == n_of[g]) umma_commit(&o_full[g]);
+            if (j + 1 < n_of[g]) {
+              // the next scores replace P: products of one CTA run in the order they are issued in
+              ok = mbar_wait(&k_full[(j + 1) % FA_KV_STAGES], ((j + 1) / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(g, j + 1);
+            }
           }
+          if (!ok) break;
           umma_commit(&v_empty[j % FA_KV_STAGES]);
-          umma_commit(o_done);
+          if (j + 1 < n_kv) umma_commit(&k_empty[(j + 1) % FA_KV_STAGES]);
         }
       }
     } else {
       // ------------------------------------------------------------------ softmax + epilogue
-      const int quarter = warp & 3;
+      const int quarter = warp & 3, g = (warp - 2) >> 2;
       const int row = quarter * 32 + lane;  // query row inside the tile = TMEM lane
       const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t s_addr = lane_addr + g * FA_BN, o_addr = lane_addr + 2 * FA_BN + g * D;
       const float c_log2 = scale * 1.4426950408889634f;
-      const int qi = q0 + row;
+      const uint64_t c2 = f2_pack(c_log2, c_log2);
+      const int r0 = q0 + g * FA_BM;
+      const int qi = r0 + row;
       const int my_limit = shift + qi;  // last key this row may see
+      const int n_my = n_of[g];
       float m_run = -INFINITY, l_run = 0.f;
       bool ok = true;
-      for (int j = 0; j < n_kv; ++j) {
-        ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
+      for (int j = 0; j < n_my; ++j) {
+        ok = mbar_wait(&s_full[g], j & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t s_addr = lane_addr + (j & 1) * FA_BN;
         const int key0 = j * FA_BN;
-        // a tile needs masking when it reaches past the diagonal of this CTA's first row or past the last key
-        const bool masked = (key0 + FA_BN - 1 > shift + q0) || (key0 + FA_BN > k_len);
+        // a tile needs masking when it reaches past the diagonal of this tile's first row or past the last key
+        const bool masked = (key0 + FA_BN - 1 > shift + r0) || (key0 + FA_BN > k_len);
         const int lim = min(my_limit, k_len - 1) - key0;  // columns <= lim are visible to this row
-        // ---- pass 1: row maximum
-        float mx = -INFINITY;
+        uint32_t r[4][32];  // the fourth quarter is read again below instead of being held (168 registers per thread are to be had)
+        auto load = [&](int c4) {
+          tmem_ld_32x32(s_addr + c4 * 32, r[c4]);
+        };
+        auto hide = [&](int c4) {
 #pragma unroll
-        for (int c4 = 0; c4 < FA_BN / 32; ++c4) {
-          uint32_t r[32];
-          tmem_ld_32x32(s_addr + c4 * 32, r);
-          tmem_ld_wait();
-          if (masked) {
+          for (int i = 0; i < 32; ++i)
+            if (c4 * 32 + i > lim) r[c4][i] = 0xff800000u;  // -infinity
+        };
+        load(3);
+        load(0);
+        tmem_ld_wait();
+        load(1);
+        load(2);
+        float mx4[4];
+        auto row_max = [&](int c4) {
+          if (masked) hide(c4);
+          mx4[c4] = __uint_as_float(r[c4][0]);
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c4 * 32 + i <= lim) mx = fmaxf(mx, __uint_as_float(r[i]));
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
-          }
-        }
-        mx *= c_log2;  // scale > 0: the maximum commutes with the scaling
+          for (int i = 1; i < 32; ++i) mx4[c4] = fmaxf(mx4[c4], __uint_as_float(r[c4][i]));
+        };
+        row_max(3);
+        row_max(0);
+        tmem_ld_wait();
+        row_max(1);
+        row_max(2);
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c_log2;  // scale > 0: the maximum commutes with the scaling
         const float m_new = fmaxf(m_run, mx);
-        bool raise = false;
         if (j == 0) {
           m_run = (m_new == -INFINITY) ? 0.f : m_new;
-        } else {
-          raise = __any_sync(0xffffffffu, m_new > m_run + 8.f);
-        }
-        const float m_use = raise ? ((m_new == -INFINITY) ? 0.f : m_new) : m_run;
-        // ---- pass 2: p = 2^(s*c - m), packed to bf16; the row sum uses the unrounded values
-        uint32_t pk[FA_BN / 2];
-        float lsum = 0.f;
+        } else if (__any_sync(0xffffffffu, m_new > m_run + 8.f)) {
+          // the scores just read came after the product of the tile before: O may be corrected
+          const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+          const float f = fa_exp2(m_run - m_use);  // <= 1
+          l_run *= f;
+#pragma unroll 1
+          for (int c4 = 0; c4 < D / 32; ++c4) {
+            uint32_t o[32];
+            tmem_ld_32x32(o_addr + c4 * 32, o);
+            tmem_ld_wait();
 #pragma unroll
-        for (int c4 = 0; c4 < FA_BN / 32; ++c4) {
-          uint32_t r[32];
-          tmem_ld_32x32(s_addr + c4 * 32, r);
-          tmem_ld_wait();
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+            tmem_st_32x32(o_addr + c4 * 32, o);
+          }
+          m_run = m_use;
+        }
+        // ---- p = 2^(s*c - m), packed to bf16; the row sum uses the unrounded values
+        const uint64_t nm = f2_pack(-m_run, -m_run);
+        uint64_t sum[2] = {0, 0};
+#pragma unroll
+        for (int c4 = 0; c4 < 4; ++c4) {
+          if (c4 == 1) load(3);  // (P takes the columns of the first two quarters only)
+          if (c4 == 3) {
+            tmem_ld_wait();
+            if (masked) hide(3);
+          }
+          uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            float p0 = fa_exp2(fmaf(__uint_as_float(r[i]), c_log2, -m_use));
-            float p1 = fa_exp2(fmaf(__uint_as_float(r[i + 1]), c_log2, -m_use));
-            if (masked) {
-              if (c4 * 32 + i > lim) p0 = 0.f;
-              if (c4 * 32 + i + 1 > lim) p1 = 0.f;
-            }
-            lsum += p0 + p1;
-            pk[c4 * 16 + (i >> 1)] = pack_bf16x2(p0, p1);
+            float p0, p1;
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(r[c4][i]), __uint_as_float(r[c4][i + 1])), c2, nm), p0, p1);
+            p0 = fa_exp2(p0);
+            p1 = fa_exp2(p1);
+            sum[(i >> 1) & 1] = f2_add(sum[(i >> 1) & 1], f2_pack(p0, p1));
+            pk[i >> 1] = pack_bf16x2(p0, p1);
           }
+          tmem_st_32x16(s_addr + c4 * 16, pk);
         }
-        // ---- the previous product has finished: P may be overwritten and O may be corrected
-        if (j > 0) {
-          ok = mbar_wait(o_done, (j - 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-          if (raise) {
-            const float f = fa_exp2(m_run - m_use);  // <= 1
-            l_run *= f;
-#pragma unroll
-            for (int c4 = 0; c4 < D / 32; ++c4) {
-              uint32_t r[32];
-              tmem_ld_32x32(lane_addr + 2 * FA_BN + c4 * 32, r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
-              tmem_st_32x32(lane_addr + 2 * FA_BN + c4 * 32, r);
-            }
-            tmem_st_wait();
-            m_run = m_use;
-          }
-        }
-        l_run += lsum;
-        // ---- P -> shared memory, canonical K-major 128B-swizzle layout: 16-byte chunk i of row r sits at (i ^ (r % 8))
-        {
-          uint8_t* prow = sP + row * 128;
-          const int sw = row & 7;
-#pragma unroll
-          for (int i = 0; i < FA_BN / 8; ++i) {
-            uint4 v = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-            *reinterpret_cast<uint4*>(prow + (i >> 3) * (FA_BM * 128) + (((i & 7) ^ sw) << 4)) = v;
-          }
-        }
-        fence_proxy_async();
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+        if (lane == 0) mbar_arrive(&p_full[g]);
+        float a, b;
+        f2_unpack(f2_add(sum[0], sum[1]), a, b);
+        l_run += a + b;
       }
-      // ---- epilogue: O / l -> bf16 -> staged through shared memory (the P buffer) -> coalesced rows of `out`
-      if (ok && n_kv > 0) {
-        ok = mbar_wait(o_done, (n_kv - 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
+      // ---- epilogue: O / l -> bf16 -> staged through shared memory (the group's Q tile) -> coalesced rows of `out`
+      if (ok && n_my > 0) {
+        ok = mbar_wait(&o_full[g], 0, cta_abort, status, ERR_WAIT_TMEM_FULL);
         ok = __all_sync(0xffffffffu, ok);
       }
-      if (ok) {
+      if (ok && r0 < q_len) {
         tc_fence_after();
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         constexpr int CH = D / 8;  // 16-byte chunks per output row
-        uint8_t* orow = sP + row * (D * 2);
+        uint8_t* stage = sQ + g * S::Q_BYTES;
+        uint8_t* orow = stage + row * (D * 2);
 #pragma unroll
         for (int c4 = 0; c4 < D / 32; ++c4) {
           uint32_t r[32];
-          if (n_kv > 0) {
-            tmem_ld_32x32(lane_addr + 2 * FA_BN + c4 * 32, r);
+          if (n_my > 0) {
+            tmem_ld_32x32(o_addr + c4 * 32, r);
             tmem_ld_wait();
           } else {
 #pragma unroll
@@ -338,13 +345,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
         if (qi < q_len && lse != nullptr)
           lse[static_cast<size_t>(h) * lse_stride + q_off + qi] = (m_run + log2f(fmaxf(l_run, 1e-38f))) * 0.6931471805599453f;
-        fa_named_barrier(1, 128);
-        const int t = threadIdx.x - 64;  // 0..127
-        const int rows_valid = min(FA_BM, q_len - q0);
+        if (g == 0) fa_named_barrier(1, 128);
+        else fa_named_barrier(2, 128);
+        const int t = (threadIdx.x - 64) & 127;
+        const int rows_valid = min(FA_BM, q_len - r0);
         for (int idx = t; idx < rows_valid * CH; idx += 128) {
           const int rr = idx / CH, ch = idx % CH;
-          const uint4 v = *reinterpret_cast<const uint4*>(sP + rr * (D * 2) + ((ch ^ (rr & (CH - 1))) << 4));
-          *reinterpret_cast<uint4*>(out + static_cast<size_t>(q_off + q0 + rr) * out_stride + h * D + ch * 8) = v;
+          const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * (D * 2) + ((ch ^ (rr & (CH - 1))) << 4));
+          *reinterpret_cast<uint4*>(out + static_cast<size_t>(q_off + r0 + rr) * out_stride + h * D + ch * 8) = v;
         }
       }
     }
@@ -374,15 +382,15 @@ static int launch_flash_fwd(const void* q, const void* k, const void* v, void* o
                                       CU_TENSOR_MAP_SWIZZLE_128B);
   auto kern = flash_fwd_kernel<D>;
   if (cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), S::TOTAL); e != cudaSuccess) return (int)e;
-  return (int)launch_pdl(kern, dim3(max_q_tiles, Hq), dim3(FA_THREADS), S::TOTAL, s, tq, tk, tv,
-                         reinterpret_cast<__nv_bfloat16*>(out), lse, seg, nseg, Hq, Hkv, out_stride, lse_stride, scale, status);
+  return (int)launch_pdl(kern, dim3(static_cast<unsigned>(max_q_tiles) * Hq), dim3(FA_THREADS), S::TOTAL, s, tq, tk, tv,
+                         reinterpret_cast<__nv_bfloat16*>(out), lse, seg, nseg, Hq, Hkv, max_q_tiles, out_stride, lse_stride, scale, status);
 }
 
 }  // namespace sb
 
 // q: [Tq, Hq, D] bf16 with row pitch q_stride (elements; the head dim is contiguous), k / v: [Tk, Hkv, D] with pitches
 // k_stride / v_stride; out: [Tq, Hq * D] with pitch out_stride; lse: [Hq, lse_stride] fp32 or null. seg: device table of
-// nseg x 4 ints (see the top of this file). max_q_tiles: an upper bound of the total number of 128-row query tiles over
+// nseg x 4 ints (see the top of this file). max_q_tiles: an upper bound of the total number of 256-row pairs of query tiles over
 // all segments (CTAs beyond the real count exit at once). Base pointers 16-byte aligned, pitches multiples of 8.
 // Returns 0, a cudaError_t value, or -1 when the head dim is not 64 or 128.
 extern "C" int sb_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* seg, int nseg,

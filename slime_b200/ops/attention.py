@@ -82,7 +82,7 @@ def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, 
         out = (torch.zeros if zero_uncovered else torch.empty)(Tq, Hq, D, dtype=q.dtype, device=q.device)
     lse = (torch.zeros if zero_uncovered else torch.empty)(Hq, Tq, dtype=torch.float32, device=q.device)
     nseg = seg.shape[0]
-    max_q_tiles = -(-Tq // 128) + nseg
+    max_q_tiles = -(-Tq // 256) + nseg  # 256 query rows per CTA
     fn = _lib.bind("sb_flash_fwd", [_lib.P] * 6 + [_lib.I] * 12 + [_lib.F, _lib.P, _lib.P])
     rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), seg.data_ptr(), nseg, max_q_tiles, Tq, Tk,
             Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), out.stride(0), Tq, float(scale),

@@ -161,3 +161,30 @@ def test_flash_backward_splits_and_tables(kernels, lens, Hq, Hkv, D):
         assert torch.equal(a, b), f"{name} is not the same twice"
         rel = float((a.float() - w).norm() / w.norm())
         assert rel < 3 * 2**-8, f"{name}: {rel}"
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("pairs", [
+    [(255, 255), (256, 256), (257, 257), (384, 384), (1, 1)],  # one tile, two whole tiles, a third one alone
+    [(1, 1000), (130, 257), (300, 301), (200, 900), (129, 129)],  # behind a context of any length
+])  # fmt: skip
+def test_flash_forward_pairs_of_tiles(kernels, pairs, D):
+    """Query tiles in pairs: the second one empty, ragged or with more key tiles than the first. Large scores make the running maximum rise.
+    Bounds: probabilities are rounded to bf16 (2^-9) and so is the output."""
+    from slime_b200.ops import _lib, attention
+
+    torch.manual_seed(D)
+    Hq, Hkv = 6, 2
+    Tq, Tk = sum(a for a, _ in pairs), sum(b for _, b in pairs)
+    q = (torch.randn(Tq, Hq, D, device="cuda") * 4).to(torch.bfloat16)
+    k, v = (torch.randn(Tk, Hkv, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    cu = lambda i: torch.tensor([0] + [p[i] for p in pairs], device="cuda").cumsum(0)  # noqa: E731
+    seg = attention.segments_extend(cu(0), cu(1))
+    out, lse = attention.flash_fwd(q, k, v, seg, D**-0.5)
+    _lib.check_status("cuda")
+    want = _ref(q, k, v, seg.cpu(), D**-0.5)
+    assert float((out.float() - want).norm() / want.norm()) < 2 * 2**-8
+    for qo, ql, ko, kl in seg.tolist():
+        s = torch.einsum("thd,shd->hts", q[qo : qo + ql].double(), k[ko : ko + kl].double().repeat_interleave(Hq // Hkv, 1)) * D**-0.5
+        s = s.masked_fill(~torch.ones(ql, kl, dtype=torch.bool, device="cuda").tril(kl - ql), -math.inf)
+        assert float((lse[:, qo : qo + ql] - s.logsumexp(-1)).abs().max()) < 1e-4 * max(1.0, float(s.amax()))
