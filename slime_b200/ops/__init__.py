@@ -7,6 +7,7 @@ silent GPU fallback: a CUDA tensor without the built library raises.
 
 from __future__ import annotations
 
+import functools
 import math
 import os
 
@@ -93,6 +94,33 @@ def _pick_splitk(M: int, N: int, K: int, bn: int, sms: int = 148) -> int:
     return max(1, min(kb // 8, sms // tiles))
 
 
+@functools.lru_cache(maxsize=4096)
+def _pick_pair(M: int, N: int, K: int, split_last: bool, sms: int = 148) -> int:
+    """Tile width of the kernel that works on pairs of SMs (``csrc/gemm_pair_sm100.cu``), 0 where the one-SM kernel is better.
+
+    A wave model again, in widths of a 256-wide tile at full rate. Measured (9198 x 19456 x 2560 and the like): pairs run a 256-wide
+    tile 1.12 times as fast as one SM; narrower tiles reach 0.92 (224 wide), 0.85 (192) and 0.65 (128) of its rate per column, and pay
+    where they fit N (896 = 4 x 224) or fill a wave. A pair's launch is about 2 us longer (two CTAs meet before and after), the
+    time of 1900 columns of one k-block: 397 x 9728 x 896 takes 22.7 us on single SMs, 23.6 on pairs; 15800 x 9728 x 896 217 and 193."""
+    kb = -(-K // 64)
+    pairs = sms // 2
+    best, width = 1e30, 0
+    for bn, rate in ((256, 1.0), (224, 0.92), (192, 0.85), (128, 0.65)):
+        tiles = -(-M // 256) * -(-N // bn)
+        if split_last and tiles >= pairs:  # with fewer tiles the uniform slices of the one-SM kernel are faster (35 and 39 us: 896 x 896 x 15800)
+            waves = tiles / pairs
+        elif split_last:
+            continue
+        else:
+            waves = -(-tiles // pairs)
+        cost = waves * bn / rate + 1900.0 / kb
+        if cost < best:
+            best, width = cost, bn
+    t128 = -(-M // 128)
+    single = min(-(-(t128 * -(-N // 256)) // sms) * 256 / 0.88, -(-(t128 * -(-N // 128)) // sms) * 128 / 0.62)
+    return width if best < single else 0
+
+
 def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, accumulate=False, bn=None, splitk=None):
     """``out (+)= op(A) @ op(B)^T (+ bias)`` with fp32 accumulation on the tcgen05 tensor cores.
 
@@ -125,6 +153,12 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
         a = a.contiguous()
     if b.stride(-1) != 1:
         b = b.contiguous()
+    if bn is None and splitk is None and (b_mn or not a_mn):
+        sms, split_last = _lib.sm_count(a.device), accumulate and not BATCH_INVARIANT
+        width = _pick_pair(M, N, K, split_last, sms)
+        res = _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms) if width else None
+        if res is not None:
+            return res
     bn = bn or _pick_bn(M, N)
     can_split = out_dtype == torch.float32 and (accumulate or (out is None and N % 4 == 0))  # TMA reduce-add: 16-byte rows
     if splitk is None:
@@ -146,6 +180,26 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
         int(accumulate), bn, int(splitk), P(_lib.status_word(a.device)), _lib.sm_count(a.device), _lib.stream(),
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_bf16")
+    return out
+
+
+def _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms):
+    """None: an output that TMA cannot write (base or pitch not a multiple of 16 bytes)."""
+    if out is None:
+        assert not accumulate
+        out = torch.empty(M, N, dtype=out_dtype, device=a.device)
+    assert out.stride(-1) == 1 and out.shape == (M, N)
+    assert not (accumulate and out.dtype != torch.float32), "accumulate needs an fp32 output"
+    lda, ldb, ldc = a.stride(0), b.stride(0), out.stride(0)
+    assert lda % 8 == 0 and ldb % 8 == 0, "TMA needs 16-byte row pitches (multiples of 8 bf16)"
+    if out.data_ptr() % 16 or (ldc * out.element_size()) % 16:
+        return None
+    f32 = out.dtype == torch.float32
+    rc = _lib.lib().sb_gemm_pair(
+        P(a), P(b), P(out), P(bias), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32), int(accumulate), width, int(split_last), 1,
+        None, None, P(_lib.status_word(a.device)), sms, _lib.stream(),
+    )  # fmt: skip
+    _lib.check(rc, "sb_gemm_pair")
     return out
 
 

@@ -70,6 +70,7 @@ _SIGS = {
     "sb_gemm_fp8_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, I, P],
     "sb_gemm_bf16_grouped": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, P],
     "sb_gemm_bf16_splitk": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, I, P],
+    "sb_gemm_pair": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, P],
     "sb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_fwd_f32x": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, I, P],

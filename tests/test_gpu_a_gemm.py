@@ -80,3 +80,27 @@ def test_fp32_output_of_any_width(kernels):
         a, b = torch.randn(7, 4096, device="cuda").bfloat16(), torch.randn(N, 4096, device="cuda").bfloat16()
         got = ops.gemm(a, b, out_dtype=torch.float32)
         torch.testing.assert_close(got, a.float() @ b.float().t(), atol=2e-2, rtol=2e-3)
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (136, 136, 72), (520, 904, 320), (9728, 896, 1096)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("width", [256, 224, 192, 160, 128])
+def test_pairs_of_sms(kernels, M, N, K, a_mn, b_mn, width):
+    """Every width and layout of the two-SM kernel: the same sums in the same order as the one-SM kernel, bit for bit; where the last
+    wave is cut along K, fp32 partial sums of the same products (half an ulp of the running sum for each of at most 74 parts)."""
+    from slime_b200.ops import _lib
+
+    torch.manual_seed(M + N + K)
+    a = torch.randn(*((K, M) if a_mn else (M, K)), device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(*((K, N) if b_mn else (N, K)), device="cuda", dtype=torch.bfloat16)
+    sms = _lib.sm_count("cuda")
+    bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
+    for dt in (torch.bfloat16, torch.float32):
+        got = ops._gemm_pair(a, b, a_mn, b_mn, bias, None, dt, False, width, False, M, N, K, sms)
+        assert torch.equal(got, ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, out_dtype=dt, bn=256, splitk=1))
+    one = ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32, bn=256, splitk=1)
+    for split in (False, True):
+        acc = torch.ones(M, N, device="cuda", dtype=torch.float32)
+        ops._gemm_pair(a, b, a_mn, b_mn, None, acc, None, True, width, split, M, N, K, sms)
+        torch.testing.assert_close(acc, one + 1.0, rtol=1e-5, atol=75 * 2.0**-24 * 4 * K**0.5)
+    _lib.check_status("cuda")
