@@ -247,14 +247,12 @@ def stacked_view(tensors: list[torch.Tensor]) -> torch.Tensor | None:
     if not all(t.is_contiguous() and t.shape == t0.shape and t.dtype == t0.dtype for t in tensors):
         return None
     step = t0.numel() * t0.element_size()
-    base = t0.data_ptr()
-    if any(t.data_ptr() != base + i * step for i, t in enumerate(tensors)):
+    base, storage = t0.data_ptr(), t0.untyped_storage()
+    # tensors of their own that an allocator happened to put side by side do not count: a view past the end of t0's storage
+    # would make torch move it
+    if any(t.data_ptr() != base + i * step for i, t in enumerate(tensors)) or base + len(tensors) * step > storage.data_ptr() + storage.nbytes():
         return None
-    try:
-        return torch.empty(0, dtype=t0.dtype, device=t0.device).set_(
-            t0.untyped_storage(), t0.storage_offset(), (len(tensors), *t0.shape))  # fmt: skip
-    except RuntimeError:  # the storage ends before the last tensor: the tensors do not share it after all
-        return None
+    return torch.empty(0, dtype=t0.dtype, device=t0.device).set_(storage, t0.storage_offset(), (len(tensors), *t0.shape))
 
 
 def _stack(weights: list[torch.Tensor]) -> torch.Tensor:

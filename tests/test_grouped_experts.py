@@ -29,6 +29,12 @@ def test_padded_layout_and_stacked_view():
     assert st is not None and st.data_ptr() == flat.data_ptr() and torch.equal(st[2], views[2])
     assert grouped.stacked_view([views[0], views[2]]) is None
     assert grouped.stacked_view([torch.randn(4, 5), torch.randn(4, 5).t().contiguous().t()]) is None
+    # neighbours in memory, each with a storage of its own
+    import numpy as np
+
+    whole = np.arange(40, dtype=np.float32)
+    apart = [torch.from_numpy(whole[i * 20 : (i + 1) * 20]).view(4, 5) for i in range(2)]
+    assert apart[1].data_ptr() == apart[0].data_ptr() + 80 and grouped.stacked_view(apart) is None
 
 
 def test_grouped_experts_module_matches_loop_on_cpu():
