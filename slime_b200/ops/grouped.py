@@ -10,8 +10,8 @@ only needs a per-tile row offset into the stacked weights (``csrc/gemm_sm100.cu`
     y = lay.unpad(grouped_linear(swiglu(h), lay, fc2_weights))
 
 Forward ``y_e = x_e W_e^T`` and the input gradient ``dx_e = dy_e W_e`` are one grouped launch each; the weight
-gradients are one ``dy_e^T x_e`` GEMM per expert over that expert's row range (accumulated straight into
-``main_grad`` when the parameter has one). The experts' weights are used in place when they are adjacent in memory (the
+gradients ``dy_e^T x_e`` are one grouped launch too where the experts' ``main_grad`` are adjacent (it adds to them),
+and one GEMM per expert over that expert's row range otherwise. The experts' weights are used in place when they are adjacent in memory (the
 flat parameter buffer lays them out that way); otherwise they are stacked with a copy.
 On CPU the same functions run a per-expert fp32 loop (the numerics oracle of the GPU path).
 """
@@ -180,6 +180,7 @@ class PaddedLayout:
         self.dest = (torch.arange(self.rows, dtype=torch.long) + shift).to(device)  # sorted row -> padded row
         tiles = torch.tensor([pc // TILE for pc in self.padded], dtype=torch.long)
         self.tile_expert = torch.repeat_interleave(torch.arange(self.num_experts), tiles).to(device=device, dtype=torch.int32)
+        self.expert_rows = torch.tensor([pstarts, self.counts], dtype=torch.int32).to(device)  # first padded row, rows
 
     def pad(self, x: torch.Tensor) -> torch.Tensor:
         return x.new_zeros(self.rows_padded, x.shape[-1]).index_copy(0, self.dest, x)
@@ -329,6 +330,26 @@ def grouped_gemm_fp8(a: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, 
     return out
 
 
+def _add_weight_grads(dy: torch.Tensor, x: torch.Tensor, lay, grads: list[torch.Tensor]) -> bool:
+    """``grads[e] += dy[rows of e]^T @ x[rows of e]`` in one launch on pairs of SMs; False where the one launch does not apply.
+
+    One GEMM per expert took 45 us of 8 k-blocks each (1536 x 2048, 512 rows), a launch whose tiles fill the SMs once and drain; one
+    launch of all is bound by reading and writing the fp32 gradients."""
+    if not dy.is_cuda or dy.dtype != torch.bfloat16 or x.dtype != torch.bfloat16 or grads[0].dtype != torch.float32:
+        return False
+    out = stacked_view(grads)
+    E, (M, N) = len(grads), grads[0].shape
+    if out is None or out.data_ptr() % 16 or M % 8 or N % 8 or lay.rows_padded == 0:
+        return False
+    width = min((256, 224, 192, 128), key=lambda bn: -(-N // bn) * bn / {256: 1.0, 224: 0.92, 192: 0.85, 128: 0.65}[bn])  # rates: ops._pick_pair
+    rc = _lib.lib().sb_gemm_pair(
+        P(dy), P(x), P(out), None, M, N, lay.rows_padded, dy.stride(0), x.stride(0), N, 1, 1, 1, 1, width, 0, E, P(lay.expert_rows[0]),
+        P(lay.expert_rows[1]), P(_lib.status_word(dy.device)), _lib.sm_count(dy.device), _lib.stream(),
+    )  # fmt: skip
+    _lib.check(rc, "sb_gemm_pair")
+    return True
+
+
 class _GroupedLinear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, lay, *weights):
@@ -344,6 +365,12 @@ class _GroupedLinear(torch.autograd.Function):
         lay, weights = ctx.lay, ctx.weights
         dy = dy.contiguous()
         dx = grouped_gemm(dy, _stack(list(weights)), lay, b_mn=True) if ctx.needs_input_grad[0] else None
+        held = [getattr(w, "main_grad", None) for w in weights]
+        if all(ctx.needs_input_grad[2:]) and all(g is not None for g in held) and _add_weight_grads(dy, x.contiguous(), lay, held):
+            for w, n in zip(weights, lay.counts):
+                if n:
+                    w.grad_added_to_main_grad = True
+            return (dx, None, *(None for _ in weights))
         dws = []
         for e, w in enumerate(weights):
             if not ctx.needs_input_grad[2 + e]:

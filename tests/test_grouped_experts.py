@@ -235,3 +235,30 @@ def test_moe_engine_decode_in_cuda_graphs_matches_eager_launches(kernels):
     assert got[0][0] == got[1][0]
     assert max(abs(a - b) for x, y in zip(got[0][1], got[1][1]) for a, b in zip(x, y)) < 1e-3
     assert all(torch.equal(a, b) for a, b in zip(got[0][2], got[1][2]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(512, 768), (264, 904), (1536, 128)])
+@pytest.mark.parametrize("counts", [[300, 0, 77, 129, 1, 128, 64, 65], [0, 0, 5], [4000, 1]])
+def test_weight_gradients_of_all_experts_in_one_launch(kernels, rows, cols, counts):
+    """Adjacent main_grads: the one launch against a GEMM per expert, on what was there before; other experts' rows stay out of it.
+    Sums of the same products in the same order: they differ by the roundings of the added fp32 parts alone."""
+    from slime_b200 import ops
+    from slime_b200.ops import _lib
+
+    torch.manual_seed(sum(counts))
+    lay = grouped.PaddedLayout(counts, "cuda")
+    x, dy = (lay.pad(torch.randn(sum(counts), n, device="cuda").bfloat16()) for n in (cols, rows))
+    flat = torch.randn(len(counts), rows, cols, device="cuda")
+    want = flat.clone()
+    for e, n in enumerate(counts):
+        s = lay.padded_starts[e]
+        if n:
+            ops.gemm(dy[s : s + n], x[s : s + n], a_mn=True, b_mn=True, out=want[e], accumulate=True, bn=128, splitk=1)
+    before = flat.clone()
+    assert grouped._add_weight_grads(dy, x, lay, [flat[e] for e in range(len(counts))])
+    _lib.check_status("cuda")
+    torch.testing.assert_close(flat, want, rtol=2**-22, atol=2**-22)
+    for e, n in enumerate(counts):
+        assert n or torch.equal(flat[e], before[e])
+    assert not grouped._add_weight_grads(dy, x, lay, [flat[e].clone() for e in range(len(counts))])  # not adjacent
