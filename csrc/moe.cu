@@ -8,6 +8,10 @@
 //                         bf16 after every route, which reproduces a chain of bf16 adds bit for bit.
 //                         This is the combine step of the forward pass and, with w = null, the gradient of the scatter.
 //   sb_moe_route_weight_grad   dw[s] = <rows[dest[s], :], dy[s / k, :]>    (gradient of the combine w.r.t. the weights)
+//   sb_moe_place_rows     out[r, :] = x[slot[r] / k, :], zero where slot[r] < 0: the scatter seen from the padded rows (trainer), which
+//                         writes each row once, padding included, instead of a fill and a copy
+//   sb_moe_combine_bwd    d_rows[r, :] = w[slot[r]] * dy[slot[r] / k, :] (zero where slot[r] < 0) and the weights' gradient of the same
+//                         slot, in one pass over `rows`
 //
 // One warp per slot (scatter, weight grad) or per token (gather); lanes stride over the row in 16-byte vectors.
 #include "common.cuh"
@@ -38,17 +42,28 @@ moe_gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restr
       float acc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-      for (int j = 0; j < k; ++j) {
-        const int d = dest[t * k + j];
-        if (d < 0) continue;
-        const float wj = w != nullptr ? w[t * k + j] : 1.f;
-        const uint4 u = reinterpret_cast<const uint4*>(rows + static_cast<long>(d) * H)[c];
-        const float2 a0 = unpack_bf16x2(u.x), a1 = unpack_bf16x2(u.y), a2 = unpack_bf16x2(u.z), a3 = unpack_bf16x2(u.w);
-        const float v[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
+      for (int j0 = 0; j0 < k; j0 += 4) {  // four routes' loads in flight, summed in order
+        uint4 u[4];
+        float wj[4];
+        int d[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          acc[i] = fmaf(wj, v[i], acc[i]);
-          if (round_each) acc[i] = __bfloat162float(__float2bfloat16(acc[i]));
+        for (int i = 0; i < 4; ++i) {
+          d[i] = j0 + i < k ? dest[t * k + j0 + i] : -1;
+          wj[i] = d[i] >= 0 && w != nullptr ? w[t * k + j0 + i] : 1.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          u[i] = d[i] >= 0 ? reinterpret_cast<const uint4*>(rows + static_cast<long>(d[i]) * H)[c] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (d[j] < 0) continue;
+          const float2 a0 = unpack_bf16x2(u[j].x), a1 = unpack_bf16x2(u[j].y), a2 = unpack_bf16x2(u[j].z), a3 = unpack_bf16x2(u[j].w);
+          const float v[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            acc[i] = fmaf(wj[j], v[i], acc[i]);
+            if (round_each) acc[i] = __bfloat162float(__float2bfloat16(acc[i]));
+          }
         }
       }
       uint4 o;
@@ -79,6 +94,66 @@ moe_route_weight_grad_kernel(const __nv_bfloat16* __restrict__ rows, const int* 
     }
     acc = warp_sum(acc);  // fixed butterfly order: the same bits on every run
     if (lane == 0) dw[s] = acc;
+  }
+}
+
+// The trainer's two row passes. Both are bound by HBM: 65.9k routes of 2048 columns in 74k padded rows write 0.3 GB (place) and read and
+// write 0.3 GB each (combine_bwd); the 34 MB of tokens stay in L2. Four vectors a lane are in flight.
+__global__ void __launch_bounds__(256)
+moe_place_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ slot, uint4* __restrict__ out, long rows, int k, int nvec) {
+  const int lane = threadIdx.x & 31;
+  for (long r = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); r < rows; r += static_cast<long>(gridDim.x) * 8) {
+    const int s = slot[r];
+    const uint4* src = x + static_cast<long>(s < 0 ? 0 : s / k) * nvec;
+    uint4* dst = out + r * nvec;
+    for (int c0 = lane; c0 < nvec; c0 += 128) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = s >= 0 && c0 + 32 * u < nvec ? src[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + 32 * u < nvec) dst[c0 + 32 * u] = v[u];
+    }
+  }
+}
+
+__device__ __forceinline__ void scale_and_dot(uint32_t r, uint32_t d, float w, uint32_t& out, float& acc) {
+  const float2 a = unpack_bf16x2(r), b = unpack_bf16x2(d);
+  acc = fmaf(a.y, b.y, fmaf(a.x, b.x, acc));
+  out = pack_bf16x2(w * b.x, w * b.y);
+}
+
+__global__ void __launch_bounds__(256)
+moe_combine_bwd_kernel(const uint4* __restrict__ rows, const int* __restrict__ slot, const float* __restrict__ w, const uint4* __restrict__ dy,
+                       uint4* __restrict__ d_rows, float* __restrict__ dw, long n, int k, int nvec) {
+  const int lane = threadIdx.x & 31;
+  for (long r = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); r < n; r += static_cast<long>(gridDim.x) * 8) {
+    const int s = slot[r];
+    const uint4* src = rows + r * nvec;
+    const uint4* g = dy + static_cast<long>(s < 0 ? 0 : s / k) * nvec;
+    uint4* dst = d_rows + r * nvec;
+    const float ws = s < 0 ? 0.f : w[s];
+    float acc = 0.f;
+    for (int c0 = lane; c0 < nvec; c0 += 128) {
+      uint4 a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = s >= 0 && c0 + 32 * u < nvec;
+        a[u] = in ? src[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
+        b[u] = in ? g[c0 + 32 * u] : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        uint4 o;
+        scale_and_dot(a[u].x, b[u].x, ws, o.x, acc);
+        scale_and_dot(a[u].y, b[u].y, ws, o.y, acc);
+        scale_and_dot(a[u].z, b[u].z, ws, o.z, acc);
+        scale_and_dot(a[u].w, b[u].w, ws, o.w, acc);
+        if (c0 + 32 * u < nvec) dst[c0 + 32 * u] = o;
+      }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && s >= 0) dw[s] = acc;
   }
 }
 
@@ -220,15 +295,16 @@ moe_topk_kernel(const float* __restrict__ logits, const float* __restrict__ shif
 
 // Expert-sorted, tile-padded layout of S = T * k routes in one launch of one CTA: every expert's rows start at a multiple
 // of 128, routes keep their order inside an expert. slot_dest[s] = padded row of route s (-1: served elsewhere),
-// tile_expert[i] = expert of the i-th 128-row tile (tiles past the last used one: the last expert).
+// tile_expert[i] = expert of the i-th 128-row tile (tiles past the last used one: the last expert). Where the trainer asks for them:
+// row_slot[r] = route in padded row r (the caller fills it with -1), expert_rows = first padded row of each expert, then rows of each.
 // Warp w owns a contiguous range of routes; two sweeps (count, place) with per-warp counters in shared memory, ranks inside
 // a warp by match_any: no atomics, so the layout is the same on every run.
 constexpr int LAYOUT_WARPS = 32;
 constexpr int LAYOUT_TILE = 128;
 constexpr int LAYOUT_AHEAD = 8;
 __global__ void __launch_bounds__(LAYOUT_WARPS * 32)
-moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int* __restrict__ tile_expert, int S, int E, int first,
-                  int tiles) {
+moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int* __restrict__ tile_expert, int* __restrict__ row_slot,
+                  int* __restrict__ expert_rows, int S, int E, int first, int tiles) {
   extern __shared__ int sm[];
   int* cnt = sm;                       // [LAYOUT_WARPS][E]
   int* pend = sm + LAYOUT_WARPS * E;   // [E] end of the expert's padded range
@@ -265,6 +341,7 @@ moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int*
       run += c;
     }
     pend[e] = (run + LAYOUT_TILE - 1) / LAYOUT_TILE * LAYOUT_TILE;
+    if (expert_rows != nullptr) expert_rows[E + e] = run;
   }
   __syncthreads();
   if (warp == 0) {  // inclusive scan of the padded sizes
@@ -299,8 +376,11 @@ moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int*
       if (e >= 0 && rank == 0) mine[e] += __popc(peers);
       __syncwarp();
       if (s < s1) slot_dest[s] = e >= 0 ? base + rank : -1;
+      if (row_slot != nullptr && e >= 0) row_slot[base + rank] = s;
     }
   }
+  if (expert_rows != nullptr)
+    for (int e = threadIdx.x; e < E; e += blockDim.x) expert_rows[e] = e > 0 ? pend[e - 1] : 0;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
     const int row = t * LAYOUT_TILE;
     int lo = 0, hi = E - 1;  // first expert whose range ends after `row`
@@ -362,12 +442,32 @@ extern "C" int sb_moe_topk(const float* logits, const float* shift, const float*
   return (int)cudaGetLastError();
 }
 
-// idx [S] int32 expert ids; experts first .. first + E - 1 live here. tiles = rows of the padded buffer / 128.
-extern "C" int sb_moe_layout(const int* idx, int* slot_dest, int* tile_expert, int S, int E, int first, int tiles, cudaStream_t s) {
+// slot [rows]: route in each padded row, negative: none. x [T, H], out [rows, H].
+extern "C" int sb_moe_place_rows(const void* x, const int* slot, void* out, long rows, int k, int H, cudaStream_t s) {
+  if (rows == 0) return 0;
+  if (H % 8 != 0 || k <= 0) return (int)cudaErrorInvalidValue;
+  sb::moe_place_rows_kernel<<<sb::moe_blocks(rows), 256, 0, s>>>((const uint4*)x, slot, (uint4*)out, rows, k, H / 8);
+  return (int)cudaGetLastError();
+}
+
+// rows, d_rows [n, H], dy [T, H], w and dw [T * k] (dw of routes without a row is left alone).
+extern "C" int sb_moe_combine_bwd(const void* rows, const int* slot, const float* w, const void* dy, void* d_rows, float* dw, long n, int k,
+                                  int H, cudaStream_t s) {
+  if (n == 0) return 0;
+  if (H % 8 != 0 || k <= 0) return (int)cudaErrorInvalidValue;
+  sb::moe_combine_bwd_kernel<<<sb::moe_blocks(n), 256, 0, s>>>((const uint4*)rows, slot, w, (const uint4*)dy, (uint4*)d_rows, dw, n, k, H / 8);
+  return (int)cudaGetLastError();
+}
+
+// idx [S] int32 expert ids; experts first .. first + E - 1 live here. tiles = rows of the padded buffer / 128. row_slot [rows of the
+// padded buffer] and expert_rows [2 * E] may be null.
+extern "C" int sb_moe_layout(const int* idx, int* slot_dest, int* tile_expert, int* row_slot, int* expert_rows, int S, int E, int first, int tiles,
+                             cudaStream_t s) {
   if (S == 0) return 0;
   const int smem = (sb::LAYOUT_WARPS + 1) * E * 4;
   if (E <= 0 || smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   if (cudaError_t e = sb::ensure_dynamic_smem(reinterpret_cast<const void*>(sb::moe_layout_kernel), 200 * 1024); e != cudaSuccess)
     return (int)e;
-  return (int)sb::launch_pdl(sb::moe_layout_kernel, dim3(1), dim3(sb::LAYOUT_WARPS * 32), smem, s, idx, slot_dest, tile_expert, S, E, first, tiles);
+  return (int)sb::launch_pdl(sb::moe_layout_kernel, dim3(1), dim3(sb::LAYOUT_WARPS * 32), smem, s, idx, slot_dest, tile_expert, row_slot,
+                             expert_rows, S, E, first, tiles);
 }

@@ -136,15 +136,21 @@ class GroupedExperts(nn.Module):
             return ops.FakeInt4STE.apply(w, self.int4_qat_group)
         return w
 
+    @property
+    def grouped(self) -> bool:
+        return self.int4_qat_group == 0 and self.use_grouped_gemm
+
+    def padded(self, x, lay):
+        """x: rows of ``lay``. One grouped launch per projection instead of a loop over experts (rows padded to the GEMM's row tile)."""
+        w1 = [getattr(self.linear_fc1, f"weight{e}") for e in range(self.num_local)]
+        w2 = [getattr(self.linear_fc2, f"weight{e}") for e in range(self.num_local)]
+        return grouped.grouped_linear(ops.swiglu(grouped.grouped_linear(x, lay, w1)), lay, w2)
+
     def forward(self, x, counts: list[int]):
         """x: [sum(counts), H] rows grouped by local expert."""
-        if self.int4_qat_group == 0 and x.shape[0] > 0 and self.use_grouped_gemm:
-            # one grouped launch per projection instead of a loop over experts (rows padded to the GEMM's row tile)
+        if self.grouped and x.shape[0] > 0:
             lay = grouped.PaddedLayout(counts, x.device)
-            w1 = [getattr(self.linear_fc1, f"weight{e}") for e in range(self.num_local)]
-            w2 = [getattr(self.linear_fc2, f"weight{e}") for e in range(self.num_local)]
-            act = ops.swiglu(grouped.grouped_linear(lay.pad(x), lay, w1))
-            return lay.unpad(grouped.grouped_linear(act, lay, w2))
+            return lay.unpad(self.padded(lay.pad(x), lay))
         outs, start = [], 0
         for e, n in enumerate(counts):
             if n == 0:
@@ -195,6 +201,11 @@ class MoELayer(nn.Module):
         probs, idx, self.aux_loss = self.router(normed)
         k = idx.shape[1]
 
+        if self.ep == 1 and self.experts.grouped and idx.numel() > 0:
+            lay = grouped.RoutedLayout(idx, cfg.num_experts)
+            rows = self.experts.padded(grouped.place_rows(normed, lay), lay)
+            return self._with_shared(grouped.combine_rows(rows, lay, probs).to(x.dtype), normed), residual
+
         # ---- permute: one row per (token, slot), sorted by global expert id (stable)
         flat_e = idx.reshape(-1)
         order = torch.argsort(flat_e, stable=True)
@@ -216,9 +227,9 @@ class MoELayer(nn.Module):
             src_e = torch.repeat_interleave(torch.arange(self.num_local, device=x.device).repeat(self.ep), recv_counts.reshape(-1),
                                             output_size=total)  # fmt: skip
             local_order = torch.argsort(src_e, stable=True)
-            grouped = recv.index_select(0, local_order)
+            here = recv.index_select(0, local_order)
             local_counts = [sum(recv_h[r][e] for r in range(self.ep)) for e in range(self.num_local)]
-            y = self.experts(grouped, local_counts)
+            y = self.experts(here, local_counts)
             back = torch.empty_like(y)
             back = back.index_copy(0, local_order, y)
             out_rows = _AllToAll.apply(back, in_splits, out_splits, group)
@@ -231,9 +242,13 @@ class MoELayer(nn.Module):
         inv = torch.empty_like(order)
         inv[order] = torch.arange(order.numel(), device=order.device)
         out = weighted.index_select(0, inv).view(T, k, H).float().sum(1).to(x.dtype)
+        return self._with_shared(out, normed), residual
+
+    def _with_shared(self, out, normed):
+        cfg = self.cfg
         if self.shared_experts is not None:
             shared = self.shared_experts.ffn(normed)
             if cfg.moe_shared_expert_gate:
                 shared = shared * torch.sigmoid(normed.float() @ self.shared_experts.gate_weight.float().t()).to(shared.dtype)
             out = out + shared
-        return out, residual
+        return out

@@ -35,7 +35,9 @@ _SIGS = {
     "sb_dp_adam_bcast": [P, P, P, P, P, I, I, I, L, L, F, F, F, F, F, F, F, F, F, P, I, P],
     "sb_group_fp8_quant_1x128": [P, P, P, P, I, I, L, L, I, P],
     "sb_moe_topk": [P, P, P, P, P, L, I, L, I, I, I, F, I, I, P],
-    "sb_moe_layout": [P, P, P, I, I, I, I, P],
+    "sb_moe_layout": [P, P, P, P, P, I, I, I, I, P],
+    "sb_moe_place_rows": [P, P, P, L, I, I, P],
+    "sb_moe_combine_bwd": [P, P, P, P, P, P, L, I, I, P],
     "sb_stream_norm": [P, I, P, I, P, P, I, P, P, I, P, P, I, P, P, I, I, I, F, F, I, P, P, P, L, L, I, P, F, I, P],
     "sb_poly_norm": [P, P, P, P, I, I, I, L, L, F, I, P],
     "sb_softcap": [P, I, L, L, F, P],

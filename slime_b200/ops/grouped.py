@@ -162,6 +162,57 @@ def combine_routes(rows, dest, weights, k: int):
     return _GatherSum.apply(rows, dest, weights, k)
 
 
+class _PlaceRows(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, lay):
+        ctx.lay = lay
+        if not (x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0):
+            return scatter_rows(x, lay.slot_dest, lay.k, lay.rows_padded)
+        out = torch.empty(lay.rows_padded, x.shape[-1], dtype=x.dtype, device=x.device)
+        rc = _lib.lib().sb_moe_place_rows(P(x.contiguous()), P(lay.row_slot), P(out), lay.rows_padded, lay.k, x.shape[-1], _lib.stream())
+        _lib.check(rc, "sb_moe_place_rows")
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        return gather_sum(g.contiguous(), ctx.lay.slot_dest, None, ctx.lay.k), None
+
+
+class _CombineRows(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, rows, lay, weights):
+        ctx.lay = lay
+        ctx.save_for_backward(rows, weights)
+        return gather_sum(rows, lay.slot_dest, weights, lay.k)
+
+    @staticmethod
+    def backward(ctx, dy):
+        rows, weights = ctx.saved_tensors
+        lay, dy = ctx.lay, dy.contiguous()
+        w = weights.reshape(-1).float().contiguous()
+        if rows.is_cuda and rows.dtype == torch.bfloat16 and rows.shape[-1] % 8 == 0:
+            rows = rows.contiguous()
+            d_rows = torch.empty_like(rows)
+            dw = torch.zeros(w.numel(), dtype=torch.float32, device=rows.device)
+            rc = _lib.lib().sb_moe_combine_bwd(P(rows), P(lay.row_slot), P(w), P(dy), P(d_rows), P(dw), rows.shape[0], lay.k, rows.shape[1], _lib.stream())
+            _lib.check(rc, "sb_moe_combine_bwd")
+        else:
+            scaled = (dy.float().repeat_interleave(lay.k, dim=0) * w[:, None]).to(dy.dtype)
+            d_rows = scatter_rows(scaled, lay.slot_dest, 1, rows.shape[0])
+            dw = route_weight_grad(rows, lay.slot_dest, dy, lay.k)
+        return d_rows, None, dw.view_as(weights).to(weights.dtype)
+
+
+def place_rows(x, lay: "RoutedLayout"):
+    """[T, H] -> [rows_padded, H]: a copy of its token in every route's row, zeros in the padding (gradient: ``gather_sum``)."""
+    return _PlaceRows.apply(x, lay)
+
+
+def combine_rows(rows, lay: "RoutedLayout", weights):
+    """[rows_padded, H], [T, k] -> [T, H]: each token's weighted sum in route order (gradients for the rows and the weights)."""
+    return _CombineRows.apply(rows, lay, weights)
+
+
 class PaddedLayout:
     """Row bookkeeping for ``counts[e]`` rows per expert, each segment starting at a multiple of 128."""
 
@@ -189,6 +240,39 @@ class PaddedLayout:
         return xp.index_select(0, self.dest)
 
 
+class RoutedLayout:
+    """The trainer's layout, from the router's choices ``idx`` [T, k] of all experts: padded rows as ``PaddedLayout`` has them, routes in
+    token order inside an expert. The row counts go to the host once (they size the activations)."""
+
+    def __init__(self, idx: torch.Tensor, num_experts: int):
+        T, self.k = idx.shape
+        self.num_experts, slots, dev = num_experts, T * self.k, idx.device
+        if idx.is_cuda and num_experts <= 1024:
+            tiles = -(-(slots + num_experts * (TILE - 1)) // TILE)
+            self.slot_dest = torch.empty(slots, dtype=torch.int32, device=dev)
+            self.tile_expert = torch.empty(tiles, dtype=torch.int32, device=dev)
+            self.row_slot = torch.full((tiles * TILE,), -1, dtype=torch.int32, device=dev)
+            self.expert_rows = torch.empty(2, num_experts, dtype=torch.int32, device=dev)
+            ids = idx.to(torch.int32).contiguous()
+            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), P(self.row_slot), P(self.expert_rows), slots,
+                                          num_experts, 0, tiles, _lib.stream())  # fmt: skip
+            _lib.check(rc, "sb_moe_layout")
+            self.padded_starts, self.counts = self.expert_rows.tolist()
+            if sum(self.counts) != slots:
+                raise IndexError(f"{slots - sum(self.counts)} of {slots} routes name no expert of 0 .. {num_experts - 1}")
+        else:
+            flat = idx.reshape(-1).long()
+            lay = PaddedLayout(torch.bincount(flat, minlength=num_experts).tolist(), dev)
+            self.padded_starts, self.counts, self.tile_expert, self.expert_rows = lay.padded_starts, lay.counts, lay.tile_expert, lay.expert_rows
+            order = torch.argsort(flat, stable=True)
+            self.slot_dest = torch.empty(slots, dtype=torch.int32, device=dev)
+            self.slot_dest[order] = lay.dest.to(torch.int32)
+            self.row_slot = torch.full((lay.rows_padded,), -1, dtype=torch.int32, device=dev)
+            self.row_slot[lay.dest] = order.to(torch.int32)
+        self.rows_padded = sum(-(-c // TILE) * TILE for c in self.counts)
+        self.tile_expert, self.row_slot = self.tile_expert[: self.rows_padded // TILE], self.row_slot[: self.rows_padded]
+
+
 class DeviceLayout:
     """The same padded layout built entirely on the device from the router's choices: no host synchronisation, static
     shapes (the row count is the worst case ``T*k + E*127`` rounded up to a tile), so it can live inside a CUDA graph.
@@ -210,7 +294,8 @@ class DeviceLayout:
             self.slot_dest = torch.empty(T * k, dtype=torch.int32, device=dev)
             self.tile_expert = torch.empty(tiles, dtype=torch.int32, device=dev)
             ids = idx.to(torch.int32).contiguous()
-            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), T * k, num_experts, first_expert, tiles, _lib.stream())
+            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), None, None, T * k, num_experts,
+                                          first_expert, tiles, _lib.stream())  # fmt: skip
             _lib.check(rc, "sb_moe_layout")
             return
         flat = idx.reshape(-1).long() - first_expert

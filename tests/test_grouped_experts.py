@@ -262,3 +262,29 @@ def test_weight_gradients_of_all_experts_in_one_launch(kernels, rows, cols, coun
     for e, n in enumerate(counts):
         assert n or torch.equal(flat[e], before[e])
     assert not grouped._add_weight_grads(dy, x, lay, [flat[e].clone() for e in range(len(counts))])  # not adjacent
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E,H", [(1, 1, 1, 8), (37, 2, 5, 136), (1000, 8, 128, 2048), (300, 3, 7, 1032)])
+def test_rows_of_routes_on_gpu_match_the_definition(kernels, T, k, E, H):
+    """Layout, placing and combining with their gradients against the CPU's; bf16 rows hold the same values, so the sums over k routes
+    differ from fp32 ones by one rounding to bf16 (2^-8 of the value) and the dot products by the order of H fp32 products."""
+    torch.manual_seed(T + H)
+    idx = torch.stack([torch.randperm(E)[:k] for _ in range(T)])
+    x, dy = torch.randn(T, H).bfloat16(), torch.randn(T, H).bfloat16()
+    w = torch.rand(T, k)
+    res = []
+    for dev in ("cpu", "cuda"):
+        lay = grouped.RoutedLayout(idx.to(dev), E)
+        xd, wd = (t.detach().clone().to(dev).requires_grad_() for t in (x, w))
+        rows = grouped.place_rows(xd, lay)
+        y = grouped.combine_rows(rows * 2, lay, wd)
+        y.backward(dy.to(dev))
+        res.append([lay.slot_dest, lay.row_slot, lay.tile_expert, lay.expert_rows, rows.detach(), y.detach(), xd.grad, wd.grad])
+        assert lay.counts == torch.bincount(idx.reshape(-1), minlength=E).tolist()
+    for a, b in zip(res[0][:5], res[1][:5]):
+        assert torch.equal(a, b.cpu())
+    for a, b, tol in zip(res[0][5:], res[1][5:], (2**-7, 2**-6, 2e-5)):
+        torch.testing.assert_close(b.cpu().float(), a.float(), rtol=tol, atol=tol * (H**0.5 if tol < 1e-3 else 1))
+    with pytest.raises(IndexError):
+        grouped.RoutedLayout(torch.full((4, 1), E, device="cuda"), E)
