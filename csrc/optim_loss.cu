@@ -194,13 +194,14 @@ dlogits_kernel(const float* __restrict__ logits, const int* __restrict__ targets
 // mode 0: PPO/GRPO clip (optional dual clip eps_c > 1), mode 1: CISPO.
 // Inputs per token: logp (new), old_logp, adv, w (loss weight: mask / normaliser).
 // Outputs: g_lp[t] = d(sum_t w_t L_t)/d logp_t, and acc[0..3] += {sum w L, sum w clipfrac, sum w (old-new), sum w}
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 pg_loss_kernel(const float* __restrict__ logp, const float* __restrict__ old_logp, const float* __restrict__ adv,
                const float* __restrict__ w, const float* __restrict__ tis, float* __restrict__ g_lp,
                float* __restrict__ per_token_loss, float* __restrict__ acc, int T, float eps_lo, float eps_hi, float eps_c,
                int mode) {
-  __shared__ float scratch[32];
-  float s_loss = 0.f, s_clip = 0.f, s_kl = 0.f, s_w = 0.f;
+  // sums of thousands of terms of either sign: in 64 bits, rounded once a block
+  __shared__ double scratch[4][32];
+  double sums[4] = {0., 0., 0., 0.};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
     const float kl = old_logp[t] - logp[t];
     const float ratio = __expf(-kl);
@@ -228,20 +229,22 @@ pg_loss_kernel(const float* __restrict__ logp, const float* __restrict__ old_log
     }
     if (per_token_loss != nullptr) per_token_loss[t] = L;
     g_lp[t] = dL * wt;
-    s_loss += L * wt;
-    s_clip += clipped * w[t];
-    s_kl += kl * w[t];
-    s_w += w[t];
+    sums[0] += static_cast<double>(L) * wt;
+    sums[1] += static_cast<double>(clipped) * w[t];
+    sums[2] += static_cast<double>(kl) * w[t];
+    sums[3] += w[t];
   }
-  s_loss = block_sum<256>(s_loss, scratch);
-  s_clip = block_sum<256>(s_clip, scratch);
-  s_kl = block_sum<256>(s_kl, scratch);
-  s_w = block_sum<256>(s_w, scratch);
-  if (threadIdx.x == 0) {
-    atomicAdd(acc + 0, s_loss);
-    atomicAdd(acc + 1, s_clip);
-    atomicAdd(acc + 2, s_kl);
-    atomicAdd(acc + 3, s_w);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    for (int o = 16; o > 0; o >>= 1) sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], o);
+    if (lane == 0) scratch[i][warp] = sums[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double v = 0.;
+    for (int i = 0; i < warps; ++i) v += scratch[threadIdx.x][i];
+    atomicAdd(acc + threadIdx.x, static_cast<float>(v));
   }
 }
 
@@ -302,9 +305,9 @@ extern "C" int sb_pg_loss(const float* logp, const float* old_logp, const float*
                           float* g_lp, float* per_token_loss, float* acc, int T, float eps_lo, float eps_hi, float eps_c,
                           int mode, cudaStream_t s) {
   if (T == 0) return 0;
-  int blocks = (T + 255) / 256;
-  if (blocks > 148) blocks = 148;
-  sb::pg_loss_kernel<<<blocks, 256, 0, s>>>(logp, old_logp, adv, w, tis, g_lp, per_token_loss, acc, T, eps_lo, eps_hi,
+  // one block adds a chunk's sums in a fixed order; more rows than a chunk has go to as many blocks as fill the SMs
+  const int blocks = T <= 16384 ? 1 : 148;
+  sb::pg_loss_kernel<<<blocks, 1024, 0, s>>>(logp, old_logp, adv, w, tis, g_lp, per_token_loss, acc, T, eps_lo, eps_hi,
                                            eps_c, mode);
   return (int)cudaGetLastError();
 }
