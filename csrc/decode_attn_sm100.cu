@@ -13,8 +13,14 @@
 //   S^T and P^T are double-buffered: K·Q^T of tile i+1 is issued before the softmax of tile i starts and V^T·P^T of
 //   tile i-1 is merged underneath it, so the tensor pipe's latency is off the critical path; three
 //   smem stages keep the next tiles' K/V in flight; ~107 KB of smem and 128 TMEM columns per CTA let two CTAs share
-//   an SM (D = 64). For D = 64 the V^T operand needs 128 rows: its upper half is pointed at the K tile that follows V in the
+//   an SM. For D = 64 the V^T operand needs 128 rows: its upper half is pointed at the K tile that follows V in the
 //   stage; those 64 accumulator rows are never read.
+//   D = 128: K and V tiles are 32 KB each. Three stages of both leave one CTA per SM, whose chain (scores -> maxima -> exp -> product) took
+//   3.0 us a tile with the copies long done (252 us a layer at 64 requests of 3068 tokens, 8 kv heads: 0.5 of the copy bandwidth). So the
+//   ring there is three HALVES, K(0) V(0) K(1) V(1) ..., which lets two CTAs share an SM: while tile i is worked on its V half is all
+//   that is resident, K(i+1) and V(i+1) are in flight in the slots of K(i) and V(i-1), both free once S^T(i) is there, and
+//   K·Q^T of tile i+1 is issued behind V^T·P^T of tile i: 155 us (decode step of six Qwen3-4B layers
+//   2.02 -> 1.57 ms).
 //   Grid = (B, Hkv, splits); with splits > 1 partial (o, m, l) go to a workspace and a small combine kernel finishes.
 //   Every mbarrier wait is bounded (2 s): on expiry the CTA records a status word, skips its output, lets in-flight
 //   copies land, frees its TMEM and returns.
@@ -41,7 +47,9 @@ struct DecSmem {
   static constexpr int P_BYTES = 2 * DA_MAXG * 128;      // P^T [16 heads, 2 chunks of 64 tokens] bf16, K-major
   static constexpr int Q_BYTES = DA_MAXG * 128 * NCH;    // [16 heads, D] bf16, K-major
   static constexpr int BAR_BYTES = 128;
-  static constexpr int TOTAL = DA_STAGES * STAGE + 2 * P_BYTES + Q_BYTES + BAR_BYTES + 1024;  // +1024: manual alignment
+  static constexpr bool HALVES = D == 128;               // ring of three halves instead of three stages
+  static constexpr int RING = HALVES ? 3 * KV_TILE : DA_STAGES * STAGE;
+  static constexpr int TOTAL = RING + 2 * P_BYTES + Q_BYTES + BAR_BYTES + 1024;  // +1024: manual alignment
   static constexpr int TMEM_COLS = 128;                  // S0 @0, S1 @32, O^T @64 (16 used of each 32)
 };
 
@@ -81,9 +89,9 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sKV = smem;
-  uint8_t* sP = smem + DA_STAGES * S::STAGE;
+  uint8_t* sP = smem + S::RING;
   uint8_t* sQ = sP + 2 * S::P_BYTES;
-  uint64_t* full_k = reinterpret_cast<uint64_t*>(sQ + S::Q_BYTES);
+  uint64_t* full_k = reinterpret_cast<uint64_t*>(sQ + S::Q_BYTES);  // ring of halves: its three barriers
   uint64_t* full_v = full_k + DA_STAGES;
   uint64_t* bar_s = full_v + DA_STAGES;
   uint64_t* bar_o = bar_s + 2;
@@ -185,13 +193,25 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   // and issues that page's boxes (one per 64-wide chunk of the head dim), so the table reads overlap. K and V have
   // separate barriers because their buffers become free at different times: K once S^T of the tile two back is done,
   // V once that tile's O^T is done. With three stages K runs three tiles ahead of the softmax and V two.
+  // buffer, barrier and phase of the K (or V) half of tile i
+  auto half_buf = [&](int i, bool is_k) -> uint8_t* {
+    if constexpr (S::HALVES) return sKV + (2 * i + (is_k ? 0 : 1)) % 3 * S::KV_TILE;
+    return sKV + i % DA_STAGES * S::STAGE + (is_k ? S::KV_TILE : 0);
+  };
+  auto half_bar = [&](int i, bool is_k) -> uint64_t* {
+    if constexpr (S::HALVES) return &full_k[(2 * i + (is_k ? 0 : 1)) % 3];
+    return is_k ? &full_k[i % DA_STAGES] : &full_v[i % DA_STAGES];
+  };
+  auto half_phase = [&](int i, bool is_k) -> uint32_t {
+    if constexpr (S::HALVES) return (2 * i + (is_k ? 0 : 1)) / 3 & 1;
+    return i / DA_STAGES & 1;
+  };
   auto issue_half = [&](int i, bool is_k) {
-    const int s = i % DA_STAGES;
     const int t0 = tile_key(i);
     const int valid = min(DA_TILE, t_end - t0);
     const int npages = (valid + page_size - 1) >> page_shift;
-    uint8_t* dst = sKV + s * S::STAGE + (is_k ? S::KV_TILE : 0);
-    uint64_t* bar = is_k ? &full_k[s] : &full_v[s];
+    uint8_t* dst = half_buf(i, is_k);
+    uint64_t* bar = half_bar(i, is_k);
     if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(npages * page_size * 128 * NCH));
     __syncwarp();
     if (lane < npages) {
@@ -206,7 +226,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   // thread 0 only: S^T[128 tok, 16] = K_tile · Q^T into S buffer (i & 1)
   auto issue_s_mma = [&](int i) {
     constexpr uint32_t idesc = make_idesc(DA_TILE, DA_MAXG, 1, 1, 0, 0);
-    const uint32_t k_addr = smem_u32(sKV + (i % DA_STAGES) * S::STAGE + S::KV_TILE);
+    const uint32_t k_addr = smem_u32(half_buf(i, true));
     const uint32_t q_addr = smem_u32(sQ);
 #pragma unroll
     for (int c = 0; c < NCH; ++c)
@@ -222,7 +242,7 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   // chunk is the K tile, whose 64 product rows are ignored.
   auto issue_o_mma = [&](int i) {
     constexpr uint32_t idesc = make_idesc(128, DA_MAXG, 1, 1, 1, 0);
-    const uint32_t v_addr = smem_u32(sKV + (i % DA_STAGES) * S::STAGE);
+    const uint32_t v_addr = smem_u32(half_buf(i, false));
     const uint32_t p_addr = smem_u32(sP + (i & 1) * S::P_BYTES);
 #pragma unroll
     for (int kc = 0; kc < 2; ++kc)
@@ -236,12 +256,18 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 
   bool ok = true;
   if (warp == 0 && ntiles > 0) {
-    for (int t = 0; t < min(ntiles, DA_STAGES); ++t) {
-      issue_half(t, true);
-      issue_half(t, false);
+    if constexpr (S::HALVES) {
+      issue_half(0, true);
+      issue_half(0, false);
+      if (ntiles > 1) issue_half(1, true);
+    } else {
+      for (int t = 0; t < min(ntiles, DA_STAGES); ++t) {
+        issue_half(t, true);
+        issue_half(t, false);
+      }
     }
     if (lane == 0) {
-      ok = mbar_wait(&full_k[0], 0, cta_abort, status, ERR_WAIT_FULL);
+      ok = mbar_wait(half_bar(0, true), 0, cta_abort, status, ERR_WAIT_FULL);
       if (ok) {
         tc_fence_after();
         issue_s_mma(0);
@@ -290,19 +316,27 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
       for (int g = 0; g < G; ++g) acc[g] = acc[g] * keep_prev[g] + __uint_as_float(r[g]) * gain_prev[g];
     }
-    if (okm && warp == 0 && j + DA_STAGES < ntiles) issue_half(j + DA_STAGES, false);
+    if constexpr (!S::HALVES)
+      if (okm && warp == 0 && j + DA_STAGES < ntiles) issue_half(j + DA_STAGES, false);
     return okm;
   };
 
   for (int i = 0; i < ntiles; ++i) {
-    const int s = i % DA_STAGES, par = i & 1;
+    const int par = i & 1;
     const int t0 = tile_key(i);
     const int valid = min(DA_TILE, t_end - t0);
     // ---- scores of this thread's token (TMEM lane = tid) for the G heads
     if (ok) ok = mbar_wait(&bar_s[par], (i >> 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
-    if (tid == 0 && ok && i + 1 < ntiles) {
+    if constexpr (S::HALVES) {
+      // S^T(i) was issued behind O^T(i-1), so both products are done: K(i)'s slot takes V(i+1), V(i-1)'s takes K(i+1) (K(1) is on its
+      // way since the start). The warp decides by itself: each of its lanes has waited on that barrier.
+      if (warp == 0 && __all_sync(0xffffffffu, ok) && i + 1 < ntiles) {
+        if (i > 0) issue_half(i + 1, true);
+        issue_half(i + 1, false);
+      }
+    } else if (tid == 0 && ok && i + 1 < ntiles) {
       // K·Q^T of the next tile goes to the other S^T buffer now, so it runs underneath this tile's softmax
-      if (mbar_wait(&full_k[(i + 1) % DA_STAGES], ((i + 1) / DA_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL)) {
+      if (mbar_wait(half_bar(i + 1, true), half_phase(i + 1, true), cta_abort, status, ERR_WAIT_FULL)) {
         tc_fence_after();
         issue_s_mma(i + 1);
       } else {
@@ -352,7 +386,8 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     ok = __syncthreads_and(ok);  // (A) tile maxima visible; everyone agrees whether to go on
     if (!ok) break;
     // S^T of this tile is complete, so nothing reads its K buffer any more: refill it for the tile two ahead
-    if (warp == 0 && i + DA_STAGES < ntiles) issue_half(i + DA_STAGES, true);
+    if constexpr (!S::HALVES)
+      if (warp == 0 && i + DA_STAGES < ntiles) issue_half(i + DA_STAGES, true);
 
     // ---- the previous tile's product is done by now (it was issued before this tile's scores were read): fold it
     //      in, which also frees O^T and the P^T buffer of two tiles ago for reuse below
@@ -380,9 +415,9 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       // Last tile: rows past the end of the sequence hold whatever the cache (or an older tile) left there.
       // Their p is 0, but 0 x NaN would poison O, so the V rows are cleared. Every thread observes the copy's
       // barrier first so that its plain stores are ordered after the TMA writes.
-      if (ok) ok = mbar_wait(&full_v[s], (i / DA_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+      if (ok) ok = mbar_wait(half_bar(i, false), half_phase(i, false), cta_abort, status, ERR_WAIT_FULL);
       if (ok && tid >= valid) {
-        uint8_t* vrow = sKV + s * S::STAGE + tid * 128;
+        uint8_t* vrow = half_buf(i, false) + tid * 128;
 #pragma unroll
         for (int c = 0; c < NCH; ++c)
 #pragma unroll
@@ -396,11 +431,19 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     if (!ok) break;
 
     if (tid == 0) {
-      if (mbar_wait(&full_v[s], (i / DA_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL)) {
+      ok = mbar_wait(half_bar(i, false), half_phase(i, false), cta_abort, status, ERR_WAIT_FULL);
+      if (ok) {
         tc_fence_after();
         issue_o_mma(i);
-      } else {
-        ok = false;
+      }
+      if constexpr (S::HALVES) {
+        if (ok && i + 1 < ntiles) {
+          ok = mbar_wait(half_bar(i + 1, true), half_phase(i + 1, true), cta_abort, status, ERR_WAIT_FULL);
+          if (ok) {
+            tc_fence_after();
+            issue_s_mma(i + 1);
+          }
+        }
       }
     }
     __syncwarp();
