@@ -17,6 +17,7 @@ import re
 import torch
 
 from slime_b200 import ops
+from slime_b200.engine import native_layer
 from slime_b200.engine.kv_cache import PagedKVCache
 from slime_b200.engine.projections import LayerProjections
 from slime_b200.engine.state_cache import RecurrentStates, StateShape
@@ -807,6 +808,7 @@ class ModelRunner:
 
             self.rope = mixers.mla_rope_table(cfg, max_context + 1, self.device)
             self.scale = mixers.mla_softmax_scale(cfg)
+        self._native_layers = native_layer.covers(self)  # prefill of fresh prompts issues a layer at a time
         self.graphs: dict[int, tuple] = {}
         self.replayed_launches = 0  # kernel-library launches executed through graph replays
         self.graph_buckets = [b for b in (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256, 384, 512) if b <= max_batch]
@@ -1282,8 +1284,11 @@ class ModelRunner:
             deepstack = embed_rows[2] if len(embed_rows) > 2 else []
         res = None
         T = ids.numel()
+        native = self._native_layers and not deepstack and native_layer.usable(self, x, positions, slots, fresh)
+        if native:
+            x, res = native_layer.prefill_layers(self, x, positions, slots, cu_q)
         recur = self._extend_recurrence(extend)
-        for li, L in enumerate(w.layers):
+        for li, L in enumerate(w.layers if not native else ()):
             if 0 < li <= len(deepstack):  # vision vectors that join the stream after layer li - 1 (stream = x + res)
                 x = x.index_add(0, embed_rows[0], deepstack[li - 1].to(x.dtype))
             normed, res = ops.rmsnorm(x, L["ln1"], cfg.norm_epsilon, res)

@@ -60,6 +60,7 @@ def _library_gemm(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate):
 
 
 # ------------------------------------------------------------------------ GEMM
+@functools.lru_cache(maxsize=4096)
 def _pick_bn(M: int, N: int, sms: int = 148) -> int:
     """Tile width by a wave model: time ~ waves x tile width / MMA efficiency (a 128-wide tile runs the tensor
     pipe at ~0.7 of a 256-wide one), waves = ceil(tiles / SMs)."""
@@ -119,6 +120,12 @@ def _pick_pair(M: int, N: int, K: int, split_last: bool, sms: int = 148) -> int:
     t128 = -(-M // 128)
     single = min(-(-(t128 * -(-N // 256)) // sms) * 256 / 0.88, -(-(t128 * -(-N // 128)) // sms) * 128 / 0.62)
     return width if best < single else 0
+
+
+def gemm_plan(M: int, N: int, K: int, f32: bool, sms: int) -> tuple[int, int, int]:
+    """What ``gemm`` does with row-major operands and a new output: (width on pairs of SMs or 0, width on one SM, slices of K)."""
+    width, bn = _pick_pair(M, N, K, False, sms), _pick_bn(M, N)
+    return width, bn, _pick_splitk(M, N, K, bn, sms) if f32 and N % 4 == 0 else 1
 
 
 def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, accumulate=False, bn=None, splitk=None):

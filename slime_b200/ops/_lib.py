@@ -73,6 +73,9 @@ _SIGS = {
     "sb_gemm_bf16_grouped": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, P],
     "sb_gemm_bf16_splitk": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, I, P],
     "sb_gemm_pair": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, P],
+    "sb_flash_fwd": [P] * 6 + [I] * 12 + [F, P, P],
+    "sb_flash_bwd": [P] * 11 + [I, P] + [I] * 17 + [F, P, P],
+    "sb_prefill_layer": [P, P],
     "sb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_fwd_f32x": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, I, P],
@@ -155,12 +158,13 @@ def ptr(t: torch.Tensor | None):
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream. ``torch.cuda.current_stream()`` builds a Stream object on the way, 6 us a call."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def check(rc: int, what: str):
+def check(rc: int, what: str, launches: int = 1):
     global _launches
-    _launches += 1
+    _launches += launches
     if rc != 0:
         detail = ""
         try:

@@ -67,6 +67,11 @@ def _strides_ok(t: torch.Tensor) -> bool:
     return t.stride(-1) == 1 and t.stride(1) == t.shape[-1] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
 
 
+def query_tiles(rows: int, nseg: int) -> int:
+    """Tiles of the forward kernel (256 query rows each) that ``nseg`` segments of ``rows`` rows in all can have at most."""
+    return -(-rows // 256) + nseg
+
+
 def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, zero_uncovered: bool = False):
     """Forward kernel launch. q [Tq, Hq, D] (heads contiguous inside a token row, any 16-byte-multiple row pitch),
     k / v [Tk, Hkv, D]. Returns ``(out [Tq, Hq, D], lse [Hq, Tq] fp32)``. The kernel writes the rows of ``out`` that
@@ -82,11 +87,12 @@ def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, 
         out = (torch.zeros if zero_uncovered else torch.empty)(Tq, Hq, D, dtype=q.dtype, device=q.device)
     lse = (torch.zeros if zero_uncovered else torch.empty)(Hq, Tq, dtype=torch.float32, device=q.device)
     nseg = seg.shape[0]
-    max_q_tiles = -(-Tq // 256) + nseg  # 256 query rows per CTA
-    fn = _lib.bind("sb_flash_fwd", [_lib.P] * 6 + [_lib.I] * 12 + [_lib.F, _lib.P, _lib.P])
-    rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), seg.data_ptr(), nseg, max_q_tiles, Tq, Tk,
-            Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), out.stride(0), Tq, float(scale),
-            _lib.ptr(_lib.status_word(q.device)), _lib.stream())  # fmt: skip
+    max_q_tiles = query_tiles(Tq, nseg)
+    rc = _lib.lib().sb_flash_fwd(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), seg.data_ptr(), nseg, max_q_tiles, Tq, Tk,
+        Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), out.stride(0), Tq, float(scale),
+        _lib.ptr(_lib.status_word(q.device)), _lib.stream(),
+    )  # fmt: skip
     _lib.check(rc, "sb_flash_fwd")
     return out, lse
 
@@ -113,11 +119,12 @@ def flash_bwd(q, k, v, o, d_o, lse, seg, scale, dq=None, dk=None, dv=None):
     k_tiles = -(-Tk // 128) + nseg
     parts = _key_parts(k_tiles * Hkv, Hq // Hkv, _lib.sm_count(q.device))
     partial = torch.empty(parts, 2, Tk, Hkv * D, dtype=torch.float32, device=q.device) if parts > 1 else None
-    fn = _lib.bind("sb_flash_bwd", [_lib.P] * 11 + [_lib.I, _lib.P] + [_lib.I] * 17 + [_lib.F, _lib.P, _lib.P])
-    rc = fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-            dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.ptr(partial), parts, seg.data_ptr(), nseg, -(-Tq // 128) + nseg, k_tiles, Tq, Tk,
-            Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dq.stride(0), dk.stride(0),
-            dv.stride(0), lse.stride(0), float(scale), _lib.ptr(_lib.status_word(q.device)), _lib.stream())  # fmt: skip
+    rc = _lib.lib().sb_flash_bwd(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(), delta.data_ptr(),
+        dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.ptr(partial), parts, seg.data_ptr(), nseg, -(-Tq // 128) + nseg, k_tiles, Tq, Tk,
+        Hq, Hkv, D, q.stride(0), k.stride(0), v.stride(0), o.stride(0), d_o.stride(0), dq.stride(0), dk.stride(0),
+        dv.stride(0), lse.stride(0), float(scale), _lib.ptr(_lib.status_word(q.device)), _lib.stream(),
+    )  # fmt: skip
     _lib.check(rc, "sb_flash_bwd")
     return dq, dk, dv
 
