@@ -387,9 +387,12 @@ rope_kv_write_kernel(__nv_bfloat16* qkv, const int* __restrict__ pos, const floa
 
 // ---------------------------------------------------------------------- SwiGLU
 // gu: [T, 2F] = [gate | up]; act[T, F] = silu(gate) * up
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, size_t T, int F) {
+// rows_used (device, or null): rows that hold anything, where T is a worst case.
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, size_t T, int F,
+                                  const int* __restrict__ rows_used) {
   pdl_wait();  // inputs come from the previous kernel in the stream
   pdl_launch_dependents();
+  if (rows_used != nullptr) T = min(T, static_cast<size_t>(__ldg(rows_used)));
   const size_t nvec = T * (F >> 3);
   for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < nvec;
        idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -539,11 +542,11 @@ static inline int ew_blocks(size_t n, int threads) {
   return (int)(b > 148 * 16 ? 148 * 16 : (b == 0 ? 1 : b));
 }
 
-extern "C" int sb_swiglu_fwd(const void* gu, void* act, long T, int F, cudaStream_t s) {
+extern "C" int sb_swiglu_fwd(const void* gu, void* act, long T, int F, const int* rows_used, cudaStream_t s) {
   if (T == 0) return 0;
   if (F % 8 != 0) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_pdl(sb::swiglu_fwd_kernel, dim3(ew_blocks((size_t)T * (F / 8), 256)), dim3(256), 0, s, (const bf16*)gu,
-                             (bf16*)act, (size_t)T, F);
+                             (bf16*)act, (size_t)T, F, rows_used);
 }
 
 extern "C" int sb_swiglu_bwd(const void* gu, const void* dact, void* dgu, long T, int F, cudaStream_t s) {

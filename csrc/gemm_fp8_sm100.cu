@@ -43,7 +43,7 @@ template <bool OUT_F32>
 __global__ void __launch_bounds__(F8_THREADS, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const float* __restrict__ sa_t, const float* __restrict__ sb, void* __restrict__ Cv, int M, int N,
-                      int K, int ldc, const int* __restrict__ tile_boff, int* status) {
+                      int K, int ldc, const int* __restrict__ tile_boff, const int* __restrict__ rows_used, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -56,8 +56,6 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + F8_BM - 1) / F8_BM, tiles_n = (N + F8_BN - 1) / F8_BN;
-  const int num_tiles = tiles_m * tiles_n;
   const int num_kb = K / F8_BK;
 
   if (threadIdx.x == 0) {
@@ -84,6 +82,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
   pdl_launch_dependents();
+  const int rows = rows_used != nullptr ? min(M, __ldg(rows_used)) : M;  // M stays the pitch of sa_t
+  const int tiles_m = (rows + F8_BM - 1) / F8_BM, tiles_n = (N + F8_BN - 1) / F8_BN;
+  const int num_tiles = tiles_m * tiles_n;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -238,9 +239,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 // A, B: e4m3 bytes, row-major with pitches lda / ldb (bytes = elements; multiples of 16). sa_t: [K/128, M] fp32.
 // sb: [ceil(N/128), K/128] fp32. C: [M, N] bf16 (out_f32 = 0) or fp32, pitch ldc elements. K must be a multiple of 128.
 // Grouped (tile_boff != nullptr): B is [num_experts * N, K], sb is [num_experts, ceil(N/128), K/128], M a multiple of 128
-// and tile_boff[M / 128] the first stack row of each row tile's expert.
+// and tile_boff[M / 128] the first stack row of each row tile's expert; rows_used as in sb_gemm_bf16_grouped.
 static int fp8_launch(const void* A, const void* B, const float* sa_t, const float* sb, void* C, int M, int N, int K, int lda,
-                      int ldb, int ldc, int out_f32, const int* tile_boff, int num_experts, int* status, int num_sms,
+                      int ldb, int ldc, int out_f32, const int* tile_boff, int num_experts, const int* rows_used, int* status, int num_sms,
                       cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (K % sb::F8_BK != 0 || lda % 16 != 0 || ldb % 16 != 0) {
@@ -264,12 +265,12 @@ static int fp8_launch(const void* A, const void* B, const float* sa_t, const flo
       e = sb::ensure_dynamic_smem(reinterpret_cast<const void*>(sb::gemm_fp8_block_kernel<true>), sb::F8_SMEM);
       if (e != cudaSuccess) return (int)e;
       e = sb::launch_pdl(sb::gemm_fp8_block_kernel<true>, dim3(grid), dim3(sb::F8_THREADS), sb::F8_SMEM, stream, tmA, tmB, sa_t,
-                         sb, C, M, N, K, ldc, tile_boff, status);
+                         sb, C, M, N, K, ldc, tile_boff, rows_used, status);
     } else {
       e = sb::ensure_dynamic_smem(reinterpret_cast<const void*>(sb::gemm_fp8_block_kernel<false>), sb::F8_SMEM);
       if (e != cudaSuccess) return (int)e;
       e = sb::launch_pdl(sb::gemm_fp8_block_kernel<false>, dim3(grid), dim3(sb::F8_THREADS), sb::F8_SMEM, stream, tmA, tmB,
-                         sa_t, sb, C, M, N, K, ldc, tile_boff, status);
+                         sa_t, sb, C, M, N, K, ldc, tile_boff, rows_used, status);
     }
     if (e != cudaSuccess) sb::set_last_error(std::string("fp8 gemm launch: ") + cudaGetErrorString(e));
     return (int)e;
@@ -282,15 +283,15 @@ static int fp8_launch(const void* A, const void* B, const float* sa_t, const flo
 extern "C" int sb_gemm_fp8_block(const void* A, const void* B, const float* sa_t, const float* sb, void* C, int M, int N,
                                  int K, int lda, int ldb, int ldc, int out_f32, int* status, int num_sms,
                                  cudaStream_t stream) {
-  return fp8_launch(A, B, sa_t, sb, C, M, N, K, lda, ldb, ldc, out_f32, nullptr, 0, status, num_sms, stream);
+  return fp8_launch(A, B, sa_t, sb, C, M, N, K, lda, ldb, ldc, out_f32, nullptr, 0, nullptr, status, num_sms, stream);
 }
 
 extern "C" int sb_gemm_fp8_grouped(const void* A, const void* B, const float* sa_t, const float* sb, void* C,
                                    const int* tile_boff, int M, int N, int K, int num_experts, int lda, int ldb, int ldc,
-                                   int out_f32, int* status, int num_sms, cudaStream_t stream) {
+                                   int out_f32, const int* rows_used, int* status, int num_sms, cudaStream_t stream) {
   if (tile_boff == nullptr) {
     sb::set_last_error("sb_gemm_fp8_grouped: needs tile_boff");
     return (int)cudaErrorInvalidValue;
   }
-  return fp8_launch(A, B, sa_t, sb, C, M, N, K, lda, ldb, ldc, out_f32, tile_boff, num_experts, status, num_sms, stream);
+  return fp8_launch(A, B, sa_t, sb, C, M, N, K, lda, ldb, ldc, out_f32, tile_boff, num_experts, rows_used, status, num_sms, stream);
 }

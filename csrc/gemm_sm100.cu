@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(GEMM_THREADS + 32 * GATHER_WARPS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, void* __restrict__ Cv, const __nv_bfloat16* __restrict__ bias,
                  int M, int N, int K, int ldc, int accumulate, int* status, const int* __restrict__ tile_boff,
-                 const __grid_constant__ Extra extra) {
+                 const int* __restrict__ rows_used, const __grid_constant__ Extra extra) {
   using S = GemmSmem<BN, STAGES>;
   constexpr int NCOLS = 2 * BN;  // two accumulator stages (power of two: 256 or 512)
   extern __shared__ uint8_t smem_raw[];
@@ -152,16 +152,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
   const int tiles_n = (N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
   const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
   // Split-K: `accumulate` carries the number of K slices in bits 8.. (1 = no split). A work item is (tile, slice); the
   // slices of a tile are summed by the epilogue's TMA reduce-add, so the caller passes a zeroed C or asks to accumulate.
   const int splitk = (accumulate >> 8) > 1 ? (accumulate >> 8) : 1;
   const bool add_out = (accumulate & 1) != 0 || splitk > 1;
   const int kb_per = (num_kb + splitk - 1) / splitk;
-  const int num_items = num_tiles * splitk;
   int rot = 0;  // first row tile of the walk
   if constexpr (Extra::kMode == 1) rot = extra.rank * (extra.rows_per_rank / GEMM_BM);
   if constexpr (Extra::kMode == 2) rot = -((extra.world << 8) | extra.rank);
@@ -192,6 +189,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   // Everything above (barriers, TMEM, descriptor prefetch) may overlap the previous kernel; operands may not.
   pdl_wait();
   pdl_launch_dependents();
+  // Grouped, rows counted on the device: A is as long as its worst case, the tiles behind the last expert's rows are left alone
+  // (12 tokens of 8 experts among 128: some 70 of 128 row tiles hold rows).
+  if (rows_used != nullptr) M = min(M, __ldg(rows_used));
+  const int tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
+  const int num_items = tiles_m * tiles_n * splitk;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -562,7 +564,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 template <int BN, int STAGES, bool A_MN, bool B_MN, bool OUT_F32, bool TMA_EPI, typename Extra = NoExtra>
 static cudaError_t launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                                int ldb, int ldc, int accumulate, int* status, int num_sms, cudaStream_t stream,
-                               const int* tile_boff = nullptr, int b_stack_rows = 0, const Extra& extra = Extra()) {
+                               const int* tile_boff = nullptr, int b_stack_rows = 0, const Extra& extra = Extra(), const int* rows_used = nullptr) {
   using S = GemmSmem<BN, STAGES>;
   // K-major operand: tensor [rows = M or N, cols = K], box [rows_tile, 64].
   // MN-major operand: tensor [rows = K, cols = M or N], box [64 k-rows, 64 cols].
@@ -594,7 +596,7 @@ static cudaError_t launch_gemm(const void* A, const void* B, void* C, const void
   if (Extra::kMode != 0) grid = num_sms;  // the collective's own work (gather pieces, owned tiles) is striped over every CTA
   constexpr int threads = Extra::kMode == 1 ? GEMM_THREADS + 32 * GATHER_WARPS : GEMM_THREADS;  // + the gather warps
   cudaError_t le = launch_pdl(kern, dim3(grid), dim3(threads), S::TOTAL, stream, tmA, tmB, tmC, C,
-                              reinterpret_cast<const __nv_bfloat16*>(bias), M, N, K, ldc, accumulate, status, tile_boff, extra);
+                              reinterpret_cast<const __nv_bfloat16*>(bias), M, N, K, ldc, accumulate, status, tile_boff, rows_used, extra);
   if (le != cudaSuccess) set_last_error(std::string("gemm launch: ") + cudaGetErrorString(le));
   return le;
 }
@@ -603,11 +605,11 @@ template <int BN, int STAGES, bool TMA_EPI>
 static cudaError_t dispatch_layout(bool a_mn, bool b_mn, bool out_f32, const void* A, const void* B, void* C,
                                    const void* bias, int M, int N, int K, int lda, int ldb, int ldc, int accumulate,
                                    int* status, int num_sms, cudaStream_t stream, const int* tile_boff = nullptr,
-                                   int b_stack_rows = 0) {
+                                   int b_stack_rows = 0, const int* rows_used = nullptr) {
 #define SB_CASE(AM, BMN, OF)                                                                                       \
   if (a_mn == AM && b_mn == BMN && out_f32 == OF)                                                                  \
     return launch_gemm<BN, STAGES, AM, BMN, OF, TMA_EPI>(A, B, C, bias, M, N, K, lda, ldb, ldc, accumulate, status, \
-                                                         num_sms, stream, tile_boff, b_stack_rows);
+                                                         num_sms, stream, tile_boff, b_stack_rows, NoExtra(), rows_used);
   SB_CASE(false, false, false)
   SB_CASE(false, false, true)
   SB_CASE(false, true, false)
@@ -670,10 +672,11 @@ extern "C" int sb_gemm_bf16_splitk(const void* A, const void* B, void* C, const 
 // segment starting at a multiple of 128 rows (the tail of a segment is padding); B is the experts' weights stacked,
 // [E * N, K] row-major (b_mn = 0, C = A * W_e^T) or [E * K, N] (b_mn = 1, C = A * W_e); tile_boff[t] (device, one int
 // per 128-row tile of A) is the first row of that tile's expert in the stack: e * N, resp. e * K. C [M, N] bf16 or fp32.
-// With b_mn = 1, K must be a multiple of 64 (a K tail would read the next expert's rows).
+// With b_mn = 1, K must be a multiple of 64 (a K tail would read the next expert's rows). rows_used (device, or null): rows of A that
+// belong to an expert; tiles past them are not computed and their rows of C not written.
 extern "C" int sb_gemm_bf16_grouped(const void* A, const void* B, void* C, const int* tile_boff, int M, int N, int K,
-                                    int num_experts, int lda, int ldb, int ldc, int b_mn, int out_f32, int bn, int* status,
-                                    int num_sms, cudaStream_t stream) {
+                                    int num_experts, int lda, int ldb, int ldc, int b_mn, int out_f32, int bn, const int* rows_used,
+                                    int* status, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (tile_boff == nullptr || num_experts <= 0 || (b_mn && K % sb::GEMM_BK != 0)) {
     sb::set_last_error("sb_gemm_bf16_grouped: needs tile_boff, num_experts > 0, and K % 64 == 0 when b_mn");
@@ -686,15 +689,15 @@ extern "C" int sb_gemm_bf16_grouped(const void* A, const void* B, void* C, const
     if (bn == 256) {
       if (tma_epi)
         return (int)sb::dispatch_layout<256, 4, true>(false, b_mn != 0, out_f32 != 0, A, B, C, nullptr, M, N, K, lda, ldb, ldc,
-                                                      0, status, num_sms, stream, tile_boff, stack_rows);
+                                                      0, status, num_sms, stream, tile_boff, stack_rows, rows_used);
       return (int)sb::dispatch_layout<256, 4, false>(false, b_mn != 0, out_f32 != 0, A, B, C, nullptr, M, N, K, lda, ldb, ldc,
-                                                     0, status, num_sms, stream, tile_boff, stack_rows);
+                                                     0, status, num_sms, stream, tile_boff, stack_rows, rows_used);
     }
     if (tma_epi)
       return (int)sb::dispatch_layout<128, 6, true>(false, b_mn != 0, out_f32 != 0, A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0,
-                                                    status, num_sms, stream, tile_boff, stack_rows);
+                                                    status, num_sms, stream, tile_boff, stack_rows, rows_used);
     return (int)sb::dispatch_layout<128, 6, false>(false, b_mn != 0, out_f32 != 0, A, B, C, nullptr, M, N, K, lda, ldb, ldc, 0,
-                                                   status, num_sms, stream, tile_boff, stack_rows);
+                                                   status, num_sms, stream, tile_boff, stack_rows, rows_used);
   } catch (const std::exception& e) {
     sb::set_last_error(e.what());
     return (int)cudaErrorInvalidValue;

@@ -13,7 +13,7 @@
 //   sb_moe_combine_bwd    d_rows[r, :] = w[slot[r]] * dy[slot[r] / k, :] (zero where slot[r] < 0) and the weights' gradient of the same
 //                         slot, in one pass over `rows`
 //
-// One warp per slot (scatter, weight grad) or per token (gather); lanes stride over the row in 16-byte vectors.
+// One warp per slot (scatter, weight grad) or per 32 vectors of a token (gather); lanes stride over the row in 16-byte vectors.
 #include "common.cuh"
 
 namespace sb {
@@ -37,8 +37,12 @@ moe_gather_sum_kernel(const __nv_bfloat16* __restrict__ rows, const int* __restr
                       __nv_bfloat16* __restrict__ y, long T, int k, int H, int round_each) {
   const int lane = threadIdx.x & 31;
   const int nvec = H >> 3;
-  for (long t = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); t < T; t += static_cast<long>(gridDim.x) * 8) {
-    for (int c = lane; c < nvec; c += 32) {
+  // a warp per (token, 32 vectors): with a warp per token the 12 tokens of a small decode batch kept 12 warps busy for 15 us
+  const int pieces = (nvec + 31) / 32;
+  for (long item = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5); item < T * pieces; item += static_cast<long>(gridDim.x) * 8) {
+    const long t = item / pieces;
+    const int c = static_cast<int>(item - t * pieces) * 32 + lane;
+    if (c < nvec) {
       float acc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -296,7 +300,8 @@ moe_topk_kernel(const float* __restrict__ logits, const float* __restrict__ shif
 // Expert-sorted, tile-padded layout of S = T * k routes in one launch of one CTA: every expert's rows start at a multiple
 // of 128, routes keep their order inside an expert. slot_dest[s] = padded row of route s (-1: served elsewhere),
 // tile_expert[i] = expert of the i-th 128-row tile (tiles past the last used one: the last expert). Where the trainer asks for them:
-// row_slot[r] = route in padded row r (the caller fills it with -1), expert_rows = first padded row of each expert, then rows of each.
+// row_slot[r] = route in padded row r (the caller fills it with -1), expert_rows = first padded row of each expert, then rows of each;
+// rows_used = rows up to the last expert's end, for kernels that leave out what lies behind.
 // Warp w owns a contiguous range of routes; two sweeps (count, place) with per-warp counters in shared memory, ranks inside
 // a warp by match_any: no atomics, so the layout is the same on every run.
 constexpr int LAYOUT_WARPS = 32;
@@ -304,7 +309,7 @@ constexpr int LAYOUT_TILE = 128;
 constexpr int LAYOUT_AHEAD = 8;
 __global__ void __launch_bounds__(LAYOUT_WARPS * 32)
 moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int* __restrict__ tile_expert, int* __restrict__ row_slot,
-                  int* __restrict__ expert_rows, int S, int E, int first, int tiles) {
+                  int* __restrict__ expert_rows, int* __restrict__ rows_used, int S, int E, int first, int tiles) {
   extern __shared__ int sm[];
   int* cnt = sm;                       // [LAYOUT_WARPS][E]
   int* pend = sm + LAYOUT_WARPS * E;   // [E] end of the expert's padded range
@@ -379,6 +384,7 @@ moe_layout_kernel(const int* __restrict__ idx, int* __restrict__ slot_dest, int*
       if (row_slot != nullptr && e >= 0) row_slot[base + rank] = s;
     }
   }
+  if (rows_used != nullptr && threadIdx.x == 0) *rows_used = pend[E - 1];
   if (expert_rows != nullptr)
     for (int e = threadIdx.x; e < E; e += blockDim.x) expert_rows[e] = e > 0 ? pend[e - 1] : 0;
   for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
@@ -416,7 +422,7 @@ extern "C" int sb_moe_gather_sum(const void* rows, const int* dest, const float*
                                  int round_each, cudaStream_t s) {
   if (T == 0) return 0;
   if (H % 8 != 0 || k <= 0) return (int)cudaErrorInvalidValue;
-  sb::moe_gather_sum_kernel<<<sb::moe_blocks(T), 256, 0, s>>>((const __nv_bfloat16*)rows, dest, w, (__nv_bfloat16*)y, T, k, H,
+  sb::moe_gather_sum_kernel<<<sb::moe_blocks(T * ((H / 8 + 31) / 32)), 256, 0, s>>>((const __nv_bfloat16*)rows, dest, w, (__nv_bfloat16*)y, T, k, H,
                                                              round_each);
   return (int)cudaGetLastError();
 }
@@ -460,14 +466,14 @@ extern "C" int sb_moe_combine_bwd(const void* rows, const int* slot, const float
 }
 
 // idx [S] int32 expert ids; experts first .. first + E - 1 live here. tiles = rows of the padded buffer / 128. row_slot [rows of the
-// padded buffer] and expert_rows [2 * E] may be null.
-extern "C" int sb_moe_layout(const int* idx, int* slot_dest, int* tile_expert, int* row_slot, int* expert_rows, int S, int E, int first, int tiles,
-                             cudaStream_t s) {
+// padded buffer], expert_rows [2 * E] and rows_used [1] may be null.
+extern "C" int sb_moe_layout(const int* idx, int* slot_dest, int* tile_expert, int* row_slot, int* expert_rows, int* rows_used, int S, int E, int first,
+                             int tiles, cudaStream_t s) {
   if (S == 0) return 0;
   const int smem = (sb::LAYOUT_WARPS + 1) * E * 4;
   if (E <= 0 || smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   if (cudaError_t e = sb::ensure_dynamic_smem(reinterpret_cast<const void*>(sb::moe_layout_kernel), 200 * 1024); e != cudaSuccess)
     return (int)e;
   return (int)sb::launch_pdl(sb::moe_layout_kernel, dim3(1), dim3(sb::LAYOUT_WARPS * 32), smem, s, idx, slot_dest, tile_expert, row_slot,
-                             expert_rows, S, E, first, tiles);
+                             expert_rows, rows_used, S, E, first, tiles);
 }

@@ -16,7 +16,7 @@ int sb_rope_kv_write(void*, const int*, const float*, const void*, const void*, 
                      cudaStream_t);
 int sb_flash_fwd(const void*, const void*, const void*, void*, float*, const int*, int, int, int, int, int, int, int, int, int, int, int, int,
                  float, int*, cudaStream_t);
-int sb_swiglu_fwd(const void*, void*, long, int, cudaStream_t);
+int sb_swiglu_fwd(const void*, void*, long, int, const int*, cudaStream_t);
 }
 
 namespace sb {
@@ -74,7 +74,7 @@ extern "C" int sb_prefill_layer(const void* layer, cudaStream_t s) {
   if (rc == 0) rc = sb_rmsnorm_fwd_f32x(p.proj, stream1, p.ln2, p.normed, p.h2, p.rstd, p.T, p.H, p.eps, s);
   if (rc != 0 || p.F == 0) return rc;
   rc = sb::project(p, 2, p.normed, p.gate_up, p.gu, nullptr, 2 * p.F, p.H, false, s);
-  if (rc == 0) rc = sb_swiglu_fwd(p.gu, p.act, p.T, p.F, s);
+  if (rc == 0) rc = sb_swiglu_fwd(p.gu, p.act, p.T, p.F, nullptr, s);
   if (rc == 0) rc = sb::project(p, 3, p.act, p.down, p.proj, nullptr, p.H, p.F, true, s);
   return rc;
 }

@@ -731,12 +731,12 @@ def _linear(x, w, bias=None, out_dtype=None, out=None):
     return quant.linear(x, w, bias=bias, out_dtype=out_dtype, out=out)
 
 
-def _grouped_linear(x, w, lay):
+def _grouped_linear(x, w, lay, rows_used=None):
     from slime_b200.ops import grouped
 
     if isinstance(w, torch.Tensor):
-        return grouped.grouped_gemm(x, w, lay)
-    return grouped.grouped_gemm_fp8(x, w.q, w.scale, lay, out_dtype=x.dtype)
+        return grouped.grouped_gemm(x, w, lay, rows_used=rows_used)
+    return grouped.grouped_gemm_fp8(x, w.q, w.scale, lay, out_dtype=x.dtype, rows_used=rows_used)
 
 
 class ModelRunner:
@@ -897,7 +897,9 @@ class ModelRunner:
         # one grouped GEMM per projection over all experts
 
         lay = grouped.DeviceLayout(idx, L["w13"].shape[0], self.w.first_expert)
-        y = lay.combine(_grouped_linear(ops.swiglu(_grouped_linear(lay.pad(x), L["w13"], lay)), L["w2"], lay), probs, x.shape[0])
+        used = lay.rows_used  # nothing is computed, or written, behind the last expert's rows
+        act = ops.swiglu_used(_grouped_linear(lay.place(x), L["w13"], lay, used), used)
+        y = lay.combine(_grouped_linear(act, L["w2"], lay, used), probs, x.shape[0])
         shared = None
         if "shared_gate_up" in L:  # always-on expert, tensor-parallel like a dense MLP
             shared = _linear(ops.swiglu(_linear(x, L["shared_gate_up"])), L["shared_down"])

@@ -486,7 +486,7 @@ class _SwiGLU(torch.autograd.Function):
         F_ = shape[-1] // 2
         g2 = gu.reshape(-1, 2 * F_).contiguous()
         act = torch.empty(g2.shape[0], F_, dtype=gu.dtype, device=gu.device)
-        _lib.check(_lib.lib().sb_swiglu_fwd(P(g2), P(act), g2.shape[0], F_, _lib.stream()), "sb_swiglu_fwd")
+        _lib.check(_lib.lib().sb_swiglu_fwd(P(g2), P(act), g2.shape[0], F_, None, _lib.stream()), "sb_swiglu_fwd")
         return act.view(*shape[:-1], F_)
 
     @staticmethod
@@ -507,6 +507,16 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gu):
     return _SwiGLU.apply(gu)
+
+
+def swiglu_used(gu, rows_used):
+    """``swiglu`` without a gradient over the first ``rows_used`` rows (a device count, or None: all); the others are left undefined."""
+    if rows_used is None or not _is_cuda(gu):
+        return swiglu(gu)
+    F_ = gu.shape[-1] // 2
+    act = torch.empty(gu.shape[0], F_, dtype=gu.dtype, device=gu.device)
+    _lib.check(_lib.lib().sb_swiglu_fwd(P(gu), P(act), gu.shape[0], F_, P(rows_used), _lib.stream()), "sb_swiglu_fwd")
+    return act
 
 
 # ------------------------------------------------------------------- embedding

@@ -35,7 +35,7 @@ _SIGS = {
     "sb_dp_adam_bcast": [P, P, P, P, P, I, I, I, L, L, F, F, F, F, F, F, F, F, F, P, I, P],
     "sb_group_fp8_quant_1x128": [P, P, P, P, I, I, L, L, I, P],
     "sb_moe_topk": [P, P, P, P, P, L, I, L, I, I, I, F, I, I, P],
-    "sb_moe_layout": [P, P, P, P, P, I, I, I, I, P],
+    "sb_moe_layout": [P, P, P, P, P, P, I, I, I, I, P],
     "sb_moe_place_rows": [P, P, P, L, I, I, P],
     "sb_moe_combine_bwd": [P, P, P, P, P, P, L, I, I, P],
     "sb_stream_norm": [P, I, P, I, P, P, I, P, P, I, P, P, I, P, P, I, I, I, F, F, I, P, P, P, L, L, I, P, F, I, P],
@@ -69,8 +69,8 @@ _SIGS = {
     "sb_moe_gather_sum": [P, P, P, P, L, I, I, I, P],
     "sb_moe_route_weight_grad": [P, P, P, P, L, I, I, P],
     "sb_gemm_fp8_block": [P, P, P, P, P, I, I, I, I, I, I, I, P, I, P],
-    "sb_gemm_fp8_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, I, P],
-    "sb_gemm_bf16_grouped": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, P],
+    "sb_gemm_fp8_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P, I, P],
+    "sb_gemm_bf16_grouped": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, I, P],
     "sb_gemm_bf16_splitk": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, I, P],
     "sb_gemm_pair": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, P],
     "sb_flash_fwd": [P] * 6 + [I] * 12 + [F, P, P],
@@ -80,7 +80,7 @@ _SIGS = {
     "sb_rmsnorm_fwd_f32x": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, I, P],
     "sb_rope": [P, P, P, P, P, P, I, I, I, I, I, I, F, F, P],
-    "sb_swiglu_fwd": [P, P, L, I, P],
+    "sb_swiglu_fwd": [P, P, L, I, P, P],
     "sb_swiglu_bwd": [P, P, P, L, I, P],
     "sb_embedding_fwd": [P, P, P, I, I, I, I, P],
     "sb_embedding_bwd": [P, P, P, I, I, I, I, P],

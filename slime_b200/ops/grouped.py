@@ -254,7 +254,7 @@ class RoutedLayout:
             self.row_slot = torch.full((tiles * TILE,), -1, dtype=torch.int32, device=dev)
             self.expert_rows = torch.empty(2, num_experts, dtype=torch.int32, device=dev)
             ids = idx.to(torch.int32).contiguous()
-            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), P(self.row_slot), P(self.expert_rows), slots,
+            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), P(self.row_slot), P(self.expert_rows), None, slots,
                                           num_experts, 0, tiles, _lib.stream())  # fmt: skip
             _lib.check(rc, "sb_moe_layout")
             self.padded_starts, self.counts = self.expert_rows.tolist()
@@ -278,8 +278,10 @@ class DeviceLayout:
     shapes (the row count is the worst case ``T*k + E*127`` rounded up to a tile), so it can live inside a CUDA graph.
 
     ``idx``: [T, k] expert ids. Rows of the padded buffer hold token ``order // k`` for the sorted assignment ``order``;
-    tiles past the last used row are zero rows attached to the last expert (they cost a little compute, nothing else).
+    tiles past the last used row are attached to the last expert; ``rows_used`` (on the device) is where they begin.
     """
+
+    rows_used = None  # CUDA layouts only
 
     def __init__(self, idx: torch.Tensor, num_experts: int, first_expert: int = 0):
         """``num_experts`` experts live here, global ids ``first_expert ...``; routes to other experts get no row
@@ -293,9 +295,10 @@ class DeviceLayout:
             tiles = self.rows_padded // TILE
             self.slot_dest = torch.empty(T * k, dtype=torch.int32, device=dev)
             self.tile_expert = torch.empty(tiles, dtype=torch.int32, device=dev)
+            self.rows_used = torch.empty(1, dtype=torch.int32, device=dev)
             ids = idx.to(torch.int32).contiguous()
-            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), None, None, T * k, num_experts,
-                                          first_expert, tiles, _lib.stream())  # fmt: skip
+            rc = _lib.lib().sb_moe_layout(P(ids), P(self.slot_dest), P(self.tile_expert), None, None, P(self.rows_used), T * k,
+                                          num_experts, first_expert, tiles, _lib.stream())  # fmt: skip
             _lib.check(rc, "sb_moe_layout")
             return
         flat = idx.reshape(-1).long() - first_expert
@@ -317,6 +320,16 @@ class DeviceLayout:
         tiles = torch.arange(self.rows_padded // TILE, device=dev) * TILE
         self.tile_expert = torch.searchsorted(pend, tiles, right=True).clamp_(max=num_experts - 1).to(torch.int32)
         self.token = self.order // k
+
+    def place(self, x: torch.Tensor) -> torch.Tensor:
+        """``pad`` with the padding left undefined: for products whose rows stand for themselves (with ``rows_used``, rows up to the
+        last expert's end are computed, and only those of routes are ever read)."""
+        if not (x.is_cuda and x.dtype == torch.bfloat16) or _checks.enabled():
+            return self.pad(x)
+        out = torch.empty(self.rows_padded, x.shape[-1], dtype=x.dtype, device=x.device)
+        rc = _lib.lib().sb_moe_scatter_rows(P(x.contiguous()), P(self.slot_dest), P(out), self.slot_dest.numel(), self.k, x.shape[-1], _lib.stream())
+        _lib.check(rc, "sb_moe_scatter_rows")
+        return out
 
     def pad(self, x: torch.Tensor) -> torch.Tensor:
         """[T, H] token activations -> [rows_padded, H] expert-sorted, zero padded."""
@@ -347,8 +360,9 @@ def _stack(weights: list[torch.Tensor]) -> torch.Tensor:
     return v if v is not None else torch.stack(datas)
 
 
-def grouped_gemm(a: torch.Tensor, w: torch.Tensor, lay, *, b_mn: bool = False, out_dtype=None) -> torch.Tensor:
-    """``out[rows of e] = a[rows of e] @ w[e]^T`` (``b_mn`` False, w [E, N, K]) or ``@ w[e]`` (``b_mn`` True, w [E, K, N])."""
+def grouped_gemm(a: torch.Tensor, w: torch.Tensor, lay, *, b_mn: bool = False, out_dtype=None, rows_used=None) -> torch.Tensor:
+    """``out[rows of e] = a[rows of e] @ w[e]^T`` (``b_mn`` False, w [E, N, K]) or ``@ w[e]`` (``b_mn`` True, w [E, K, N]).
+    ``rows_used`` (device count, or None: all): rows in tiles behind it may be left undefined."""
     E, R, C = w.shape
     M, K = a.shape
     N = C if b_mn else R
@@ -376,13 +390,13 @@ def grouped_gemm(a: torch.Tensor, w: torch.Tensor, lay, *, b_mn: bool = False, o
 
     rc = _lib.lib().sb_gemm_bf16_grouped(
         P(a), P(w), P(out), P(boff), M, N, K, E, a.stride(0), w.stride(1), out.stride(0), int(b_mn),
-        int(out_dtype == torch.float32), _pick_bn(M, N), P(_lib.status_word(a.device)), _lib.sm_count(a.device), _lib.stream(),
+        int(out_dtype == torch.float32), _pick_bn(M, N), P(rows_used), P(_lib.status_word(a.device)), _lib.sm_count(a.device), _lib.stream(),
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_bf16_grouped")
     return out
 
 
-def grouped_gemm_fp8(a: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, lay, out_dtype=torch.bfloat16) -> torch.Tensor:
+def grouped_gemm_fp8(a: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, lay, out_dtype=torch.bfloat16, rows_used=None) -> torch.Tensor:
     """``out[rows of e] = a[rows of e] @ dequant(w_q[e], w_scale[e])^T`` for block-quantised expert weights.
 
     ``a`` [rows_padded, K] bf16 is quantised here to e4m3 with one scale per row and 128-wide K group; ``w_q`` [E, N, K]
@@ -409,7 +423,7 @@ def grouped_gemm_fp8(a: torch.Tensor, w_q: torch.Tensor, w_scale: torch.Tensor, 
     boff = lay.tile_expert * N
     rc = _lib.lib().sb_gemm_fp8_grouped(
         P(a_q), P(w_q), P(a_st), P(w_scale), P(out), P(boff), M, N, K, E, a_q.stride(0), w_q.stride(1), out.stride(0),
-        int(out_dtype == torch.float32), P(_lib.status_word(a.device)), _lib.sm_count(a.device), _lib.stream(),
+        int(out_dtype == torch.float32), P(rows_used), P(_lib.status_word(a.device)), _lib.sm_count(a.device), _lib.stream(),
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_fp8_grouped")
     return out

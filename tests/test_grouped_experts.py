@@ -288,3 +288,31 @@ def test_rows_of_routes_on_gpu_match_the_definition(kernels, T, k, E, H):
         torch.testing.assert_close(b.cpu().float(), a.float(), rtol=tol, atol=tol * (H**0.5 if tol < 1e-3 else 1))
     with pytest.raises(IndexError):
         grouped.RoutedLayout(torch.full((4, 1), E, device="cuda"), E)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,k,E,fp8", [(1, 1, 4, False), (12, 8, 128, False), (12, 8, 128, True), (300, 2, 3, False), (9, 2, 8, True)])
+def test_rows_behind_the_last_expert_are_left_out(kernels, T, k, E, fp8):
+    """The engine's expert MLP over the used rows only, on buffers full of NaN, against zero padding and all rows: the same bits."""
+    from slime_b200 import ops
+    from slime_b200.engine import model_runner, quant
+
+    torch.manual_seed(T + E)
+    H, F = 256, 384
+    idx = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).cuda()
+    x, probs = torch.randn(T, H, device="cuda").bfloat16(), torch.rand(T, k, device="cuda")
+    w13, w2 = ((torch.randn(E, n, m, device="cuda") * 0.1).bfloat16() for n, m in ((2 * F, H), (H, F)))
+    if fp8:
+        w13, w2 = (quant.Fp8Weight(*w.shape, device="cuda") for w in (w13, w2))
+        for w in (w13, w2):
+            w.fill_random_(0.1)
+    lay = grouped.DeviceLayout(idx, E)
+    counts = torch.bincount(idx.reshape(-1), minlength=E)
+    assert int(lay.rows_used) == int(((counts + 127) // 128 * 128).sum())
+    lin = model_runner._grouped_linear
+    want = lay.combine(lin(ops.swiglu(lin(lay.pad(x), w13, lay)), w2, lay), probs, T)
+    junk = [torch.full((n,), float("nan"), device="cuda") for n in (1 << 16, 1 << 18, 1 << 20, 1 << 22, 1 << 23, 1 << 24, 1 << 24)]
+    del junk  # what the next buffers are made of
+    used = lay.rows_used
+    got = lay.combine(lin(ops.swiglu_used(lin(lay.place(x), w13, lay, used), used), w2, lay, used), probs, T)
+    assert torch.equal(got, want)
