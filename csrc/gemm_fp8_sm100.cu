@@ -158,18 +158,19 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       // grouped: the expert's own scale table ([ceil(N/128), K/128] per expert)
       const int expert = tile_boff != nullptr ? __ldg(tile_boff + m0 / F8_BM) / N : 0;
       const float* sb_row = sb + (static_cast<size_t>(expert) * ((N + 127) / 128) + nblk) * num_kb;
-      float c[HALF];
+      uint64_t c2[HALF / 2];  // accumulators in pairs: two multiply-adds per instruction
 #pragma unroll
-      for (int i = 0; i < HALF; ++i) c[i] = 0.f;
+      for (int i = 0; i < HALF / 2; ++i) c2[i] = 0;
       // the scales of a K block are fetched two blocks ahead: a global load issued inside the iteration that needs it
       // would put its full latency on the critical path of every block
-      auto load_scale = [&](int kb) -> float {
-        if (kb >= num_kb) return 0.f;
-        return (row < M ? __ldg(sa_t + static_cast<size_t>(kb) * M + row) : 0.f) * __ldg(sb_row + kb);
+      auto load_scale = [&](int kb) -> float2 {  // of the row and of the block; multiplied where they are used, not where they are awaited
+        if (kb >= num_kb) return make_float2(0.f, 0.f);
+        return make_float2(row < M ? __ldg(sa_t + static_cast<size_t>(kb) * M + row) : 0.f, __ldg(sb_row + kb));
       };
-      float s_cur = load_scale(0), s_next = load_scale(1);
+      float2 s_cur = load_scale(0), s_next = load_scale(1);
       for (int kb = 0; kb < num_kb; ++kb) {
-        const float s = s_cur;
+        const float s = s_cur.x * s_cur.y;
+        const uint64_t s2 = f2_pack(s, s);
         s_cur = s_next;
         s_next = load_scale(kb + 2);
         ok = mbar_wait(&acc_full[acc], acc_phase, cta_abort, status, ERR_WAIT_TMEM_FULL);
@@ -177,16 +178,18 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (!ok) break;
         tc_fence_after();
         const uint32_t t = tmem_base + acc * F8_BN + h * HALF + (static_cast<uint32_t>(q * 32) << 16);
+        // Two products per instruction, and both loads of a pass in flight before the wait. 3465 x 2560 x 9728: 156 -> 115 us (single
+        // products: 156; one load at a time, the accumulator back earlier: 170).
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
           uint32_t r0[32], r1[32];
-          tmem_ld_32x32(t + pass * 64, r0);  // both loads in flight before the wait
+          tmem_ld_32x32(t + pass * 64, r0);
           tmem_ld_32x32(t + pass * 64 + 32, r1);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            c[pass * 64 + i] = fmaf(__uint_as_float(r0[i]), s, c[pass * 64 + i]);
-            c[pass * 64 + 32 + i] = fmaf(__uint_as_float(r1[i]), s, c[pass * 64 + 32 + i]);
+          for (int i = 0; i < 16; ++i) {
+            c2[pass * 32 + i] = f2_fma(f2_pack(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1])), s2, c2[pass * 32 + i]);
+            c2[pass * 32 + 16 + i] = f2_fma(f2_pack(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1])), s2, c2[pass * 32 + 16 + i]);
           }
         }
         tc_fence_before();
@@ -198,6 +201,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       }
       const int col0 = n0 + h * HALF;
+      float c[HALF];
+#pragma unroll
+      for (int i = 0; i < HALF / 2; ++i) f2_unpack(c2[i], c[2 * i], c[2 * i + 1]);
       if (ok && row < M && col0 < N) {
         if constexpr (OUT_F32) {
           float* dst = static_cast<float*>(Cv) + static_cast<size_t>(row) * ldc + col0;
