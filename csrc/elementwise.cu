@@ -154,13 +154,23 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// dw[c] (+)= sum_p dw_partial[p, c]
-__global__ void rmsnorm_dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int P, int H,
-                                         int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
+// dw[c] (+)= sum_p dw_partial[p, c]: 32 columns a block, eight interleaved runs of rows, added up in a fixed order. One thread per column
+// walked the rows with one load in flight after the other (296 rows of 896: 12 -> 5 us).
+constexpr int DW_THREADS = 256;
+inline int dw_reduce_blocks(int H) { return (H + 31) / 32; }
+__global__ void __launch_bounds__(DW_THREADS)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int P, int H, int accumulate) {
+  __shared__ float sums[8][32];
+  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int p = 0; p < P; ++p) s += part[static_cast<size_t>(p) * H + c];
+  if (c < H)
+#pragma unroll 8
+    for (int p = run; p < P; p += 8) s += part[static_cast<size_t>(p) * H + c];
+  sums[run][lane] = s;
+  __syncthreads();
+  if (run != 0 || c >= H) return;
+#pragma unroll
+  for (int r = 1; r < 8; ++r) s += sums[r][lane];
   dw[c] = accumulate ? dw[c] + s : s;
 }
 
@@ -260,7 +270,7 @@ static cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat
     rmsnorm_bwd_warp_kernel<4><<<num_ctas, NORM_THREADS, 0, s>>>(dy, h, w, rstd, dres_in, dh, dw_partial, T, H);
   else
     rmsnorm_bwd_kernel<<<num_ctas, NORM_THREADS, 0, s>>>(dy, h, w, rstd, dres_in, dh, dw_partial, T, H);
-  rmsnorm_dw_reduce_kernel<<<(H + 255) / 256, 256, 0, s>>>(dw_partial, dw, num_ctas, H, accumulate_dw);
+  rmsnorm_dw_reduce_kernel<<<dw_reduce_blocks(H), DW_THREADS, 0, s>>>(dw_partial, dw, num_ctas, H, accumulate_dw);
   return cudaGetLastError();
 }
 
@@ -271,21 +281,75 @@ static cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat
 //   o[i] = a[i] cos - a[i+D/2] sin ; o[i+D/2] = a[i+D/2] cos + a[i] sin
 // with a = x or rmsnorm_D(x) * nw when nw != nullptr. cos/sin table: [max_pos, D/2] fp32.
 // `sign` = +1 forward rotation, -1 inverse rotation (backward of RoPE).
+// A group of D / 16 lanes has a head: each lane eight neighbouring elements of its lower half and the eight they are turned with, as
+// 16-byte accesses. Bound by HBM; with a warp per head and 2-byte accesses the instructions bound it (15800 tokens, 14 heads of 64:
+// 50 -> 8 us). VEC = false is that form, for rows that are no whole 16-byte pieces.
 template <int D>
+__device__ __forceinline__ float head_sum(float v) {  // over the lanes of a head
+#pragma unroll
+  for (int o = D / 32; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// (per-head RMSNorm and) rotation of one head's lane: lo / hi hold its sixteen elements; returns 1 / rms.
+template <int D>
+__device__ __forceinline__ float turn_head(float (&lo)[8], float (&hi)[8], const __nv_bfloat16* nw, const float* cs, int i0, float eps,
+                                           float sign) {
+  float rs = 1.f;
+  if (nw != nullptr) {
+    float ss = 0.f, g[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += lo[i] * lo[i] + hi[i] * hi[i];
+    rs = rsqrtf(head_sum<D>(ss) / D + eps);
+    load8(nw + i0, g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) lo[i] = lo[i] * rs * g[i];
+    load8(nw + D / 2 + i0, g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) hi[i] = hi[i] * rs * g[i];
+  }
+  float c[8], sn[8];
+  load8(cs + i0, c);
+  load8(cs + D / 2 + i0, sn);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float a = lo[i], b = hi[i], s = sign * sn[i];
+    lo[i] = a * c[i] - b * s;
+    hi[i] = b * c[i] + a * s;
+  }
+  return rs;
+}
+
+template <int D, bool VEC>
 __global__ void __launch_bounds__(128)
-rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* out /* may alias x: a warp reads its head fully before writing */,
+rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* out /* may alias x: a head is read fully before it is written */,
             const int* __restrict__ pos,
             const float* __restrict__ cos_sin, const __nv_bfloat16* __restrict__ nw, float* __restrict__ rstd_out,
             int T, int nheads, int head0, int in_stride, int out_stride, float eps, float sign) {
   constexpr int PER = D / 64;  // each lane handles PER pairs (i, i + D/2) ... D/2 / 32 lanes
+  constexpr int LANES = VEC ? D / 16 : 32;
   pdl_wait();  // inputs come from the previous kernel in the stream
   pdl_launch_dependents();
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long unit = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) / LANES;
   const int lane = threadIdx.x & 31;
-  if (warp_global >= T * nheads) return;
-  const int t = warp_global / nheads, hh = warp_global % nheads;
+  const bool in = unit < static_cast<long>(T) * nheads;
+  if (!VEC && !in) return;
+  const long at = in ? unit : 0;  // surplus lanes of a warp keep its shuffles whole
+  const int t = static_cast<int>(at / nheads), hh = static_cast<int>(at % nheads);
   const __nv_bfloat16* src = x + static_cast<size_t>(t) * in_stride + static_cast<size_t>(head0 + hh) * D;
   __nv_bfloat16* dst = out + static_cast<size_t>(t) * out_stride + static_cast<size_t>(head0 + hh) * D;
+  if constexpr (VEC) {
+    const int i0 = lane % LANES * 8;
+    float lo[8], hi[8];
+    load8(src + i0, lo);
+    load8(src + D / 2 + i0, hi);
+    const float rs = turn_head<D>(lo, hi, nw, cos_sin + static_cast<size_t>(pos[t]) * D, i0, eps, sign);
+    if (!in) return;
+    if (nw != nullptr && rstd_out != nullptr && i0 == 0) rstd_out[static_cast<size_t>(t) * nheads + hh] = rs;
+    store8(dst + i0, lo);
+    store8(dst + D / 2 + i0, hi);
+    return;
+  }
   float lo[PER], hi[PER];
   float ss = 0.f;
 #pragma unroll
@@ -316,13 +380,96 @@ rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* out /* may alias x: a warp re
   }
 }
 
+// Backward of per-head RMSNorm and rotation, in place on the gradients of the rotated heads: d [T, heads, D] rows of `stride`, x the
+// heads before the norm. dx = rs * (g - xhat * mean(g * xhat)) with g = inverse rotation of d, times the norm's weight; each block adds up
+// the weights' gradient of its q heads (part[block][0]) and k heads (part[block][1]). Passes of their own for the inverse rotation, 1 / rms,
+// the norm's backward and four copies between strided and packed heads
+// took 0.9 ms a layer of 9198 tokens, 32 + 8 heads of 128; this 76 us.
+template <int D>
+__global__ void __launch_bounds__(256)
+rope_norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ d, const int* __restrict__ pos,
+                     const float* __restrict__ cos_sin, const __nv_bfloat16* __restrict__ q_nw, const __nv_bfloat16* __restrict__ k_nw,
+                     float* __restrict__ part, int T, int Hq, int Hkv, int x_stride, int d_stride, float eps) {
+  constexpr int LANES = D / 16;
+  constexpr int UNITS = 256 / LANES;  // heads of a block at a time
+  __shared__ float sums[256][17];     // 17: the lanes of a head land in different banks
+  const int sub = threadIdx.x / LANES, i0 = threadIdx.x % LANES * 8;
+#pragma unroll 1
+  for (int kind = 0; kind < 2; ++kind) {
+    const __nv_bfloat16* nw = kind == 0 ? q_nw : k_nw;
+    const int heads = kind == 0 ? Hq : Hkv, head0 = kind == 0 ? 0 : Hq;
+    const long n = static_cast<long>(T) * heads;
+    float glo[8], ghi[8], wlo[8], whi[8];
+    load8(nw + i0, glo);
+    load8(nw + D / 2 + i0, ghi);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wlo[i] = whi[i] = 0.f;
+    for (long u0 = static_cast<long>(blockIdx.x) * UNITS; u0 < n; u0 += static_cast<long>(gridDim.x) * UNITS) {
+      const long u = min(u0 + sub, n - 1);  // surplus lanes keep the shuffles whole
+      const bool in = u0 + sub < n;
+      const int t = static_cast<int>(u / heads), h = head0 + static_cast<int>(u % heads);
+      const __nv_bfloat16* xs = x + static_cast<size_t>(t) * x_stride + static_cast<size_t>(h) * D;
+      __nv_bfloat16* ds = d + static_cast<size_t>(t) * d_stride + static_cast<size_t>(h) * D;
+      const float* cs = cos_sin + static_cast<size_t>(pos[t]) * D;
+      float xl[8], xh[8], dl[8], dh[8], c[8], sn[8];
+      load8(xs + i0, xl);
+      load8(xs + D / 2 + i0, xh);
+      load8(ds + i0, dl);
+      load8(ds + D / 2 + i0, dh);
+      load8(cs + i0, c);
+      load8(cs + D / 2 + i0, sn);
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ss += xl[i] * xl[i] + xh[i] * xh[i];
+      const float rs = rsqrtf(head_sum<D>(ss) / D + eps);
+      float dot = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float a = dl[i] * c[i] + dh[i] * sn[i], b = dh[i] * c[i] - dl[i] * sn[i];
+        xl[i] *= rs;
+        xh[i] *= rs;
+        if (in) {
+          wlo[i] += a * xl[i];
+          whi[i] += b * xh[i];
+        }
+        dl[i] = a * glo[i];
+        dh[i] = b * ghi[i];
+        dot += dl[i] * xl[i] + dh[i] * xh[i];
+      }
+      dot = head_sum<D>(dot) / D;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        dl[i] = rs * (dl[i] - xl[i] * dot);
+        dh[i] = rs * (dh[i] - xh[i] * dot);
+      }
+      if (in) {
+        store8(ds + i0, dl);
+        store8(ds + D / 2 + i0, dh);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      sums[threadIdx.x][i] = wlo[i];
+      sums[threadIdx.x][8 + i] = whi[i];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < D; e += 256) {
+      const int half = e / (D / 2), r = e % (D / 2);
+      float v = 0.f;
+      for (int k = 0; k < UNITS; ++k) v += sums[k * LANES + r / 8][half * 8 + r % 8];
+      part[(static_cast<size_t>(blockIdx.x) * 2 + kind) * D + e] = v;
+    }
+    __syncthreads();
+  }
+}
+
 // Inference form of the above, fused with the KV-cache write: one launch per layer instead of four. One warp per
 // (token, head) of a packed qkv row [T, (Hq + 2 Hkv) * D]:
 //   q heads  (per-head RMSNorm +) RoPE in place
 //   k heads  the same, written in place (prefill attends over the row itself) and to k_cache[slot[t], head]
 //   v heads  copied to v_cache[slot[t], head]
 // Caches are [slots, Hkv, D] contiguous; a negative slot skips the cache write (padding rows).
-template <int D>
+template <int D, bool VEC>
 __global__ void __launch_bounds__(128)
 rope_kv_write_kernel(__nv_bfloat16* qkv, const int* __restrict__ pos, const float* __restrict__ cos_sin,
                      const __nv_bfloat16* __restrict__ q_nw, const __nv_bfloat16* __restrict__ k_nw,
@@ -332,8 +479,39 @@ rope_kv_write_kernel(__nv_bfloat16* qkv, const int* __restrict__ pos, const floa
   pdl_wait();
   pdl_launch_dependents();
   const int heads = Hq + 2 * Hkv;
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  if constexpr (VEC) {  // as in rope_kernel
+    constexpr int LANES = D / 16;
+    const long unit = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) / LANES;
+    const bool in = unit < static_cast<long>(T) * heads;
+    const long at = in ? unit : 0;
+    const int t = static_cast<int>(at / heads), h = static_cast<int>(at % heads), i0 = lane % LANES * 8;
+    __nv_bfloat16* row = qkv + static_cast<size_t>(t) * row_stride + static_cast<size_t>(h) * D;
+    const int slot = h >= Hq ? slots[t] : -1;
+    const bool is_v = h >= Hq + Hkv;
+    const uint4 raw_lo = *reinterpret_cast<const uint4*>(row + i0), raw_hi = *reinterpret_cast<const uint4*>(row + D / 2 + i0);
+    float lo[8], hi[8];
+    unpack8(raw_lo, lo);
+    unpack8(raw_hi, hi);
+    turn_head<D>(lo, hi, h >= Hq ? k_nw : q_nw, cos_sin + static_cast<size_t>(pos[t]) * D, i0, eps, 1.f);
+    if (!in) return;
+    if (is_v) {
+      if (slot < 0) return;
+      __nv_bfloat16* dst = v_cache + (static_cast<size_t>(slot) * Hkv + (h - Hq - Hkv)) * D;
+      *reinterpret_cast<uint4*>(dst + i0) = raw_lo;
+      *reinterpret_cast<uint4*>(dst + D / 2 + i0) = raw_hi;
+      return;
+    }
+    store8(row + i0, lo);
+    store8(row + D / 2 + i0, hi);
+    if (slot >= 0) {
+      __nv_bfloat16* dst = k_cache + (static_cast<size_t>(slot) * Hkv + (h - Hq)) * D;
+      store8(dst + i0, lo);
+      store8(dst + D / 2 + i0, hi);
+    }
+    return;
+  }
+  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (warp_global >= T * heads) return;
   const int t = warp_global / heads, h = warp_global % heads;
   __nv_bfloat16* row = qkv + static_cast<size_t>(t) * row_stride + static_cast<size_t>(h) * D;
@@ -500,23 +678,39 @@ extern "C" int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
                                      (bf16*)dh, dw_partial, dw, T, H, num_ctas, accumulate_dw, s);
 }
 
+// Rows of whole 16-byte pieces: pointers and pitch (head widths are multiples of 64).
+static inline bool rope_vec(const void* x, int stride, const void* nw, const float* cos_sin) {
+  return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(nw) | reinterpret_cast<uintptr_t>(cos_sin)) & 15) == 0 && stride % 8 == 0;
+}
+static inline unsigned rope_blocks(long heads, int lanes) { return static_cast<unsigned>((heads * lanes + 127) / 128); }
+
 extern "C" int sb_rope(const void* x, void* out, const int* pos, const float* cos_sin, const void* nw, float* rstd,
                        int T, int nheads, int head0, int in_stride, int out_stride, int D, float eps, float sign,
                        cudaStream_t s) {
   if (T == 0 || nheads == 0) return 0;
-  const long warps = (long)T * nheads;
-  const int blocks = (int)((warps * 32 + 127) / 128);
-  if (D == 64)
-    return (int)sb::launch_pdl(sb::rope_kernel<64>, dim3(blocks), dim3(128), 0, s, (const bf16*)x, (bf16*)out, pos, cos_sin,
-                               (const bf16*)nw, rstd, T, nheads, head0, in_stride, out_stride, eps, sign);
-  else if (D == 128)
-    return (int)sb::launch_pdl(sb::rope_kernel<128>, dim3(blocks), dim3(128), 0, s, (const bf16*)x, (bf16*)out, pos, cos_sin,
-                               (const bf16*)nw, rstd, T, nheads, head0, in_stride, out_stride, eps, sign);
-  else if (D == 256)
-    return (int)sb::launch_pdl(sb::rope_kernel<256>, dim3(blocks), dim3(128), 0, s, (const bf16*)x, (bf16*)out, pos, cos_sin,
-                               (const bf16*)nw, rstd, T, nheads, head0, in_stride, out_stride, eps, sign);
-  else
+  const bool vec = rope_vec(x, in_stride, nw, cos_sin) && rope_vec(out, out_stride, nullptr, nullptr);
+#define SB_ROPE(DV, V)                                                                                                     \
+  if (D == DV && vec == V)                                                                                                 \
+    return (int)sb::launch_pdl(sb::rope_kernel<DV, V>, dim3(rope_blocks((long)T * nheads, V ? DV / 16 : 32)), dim3(128), 0, s, (const bf16*)x, \
+                               (bf16*)out, pos, cos_sin, (const bf16*)nw, rstd, T, nheads, head0, in_stride, out_stride, eps, sign);
+  SB_ROPE(64, true) SB_ROPE(64, false) SB_ROPE(128, true) SB_ROPE(128, false) SB_ROPE(256, true) SB_ROPE(256, false)
+#undef SB_ROPE
+  return (int)cudaErrorInvalidValue;
+}
+
+// x [T, (Hq + 2 Hkv) * D] before norm and rotation, d the gradients of the rotated q and k heads, turned into those of x in place (pitches
+// x_stride, d_stride). part: [blocks, 2, D] fp32 scratch; dw [2, D]: gradients of the two norms' weights, overwritten. 16-byte aligned rows.
+extern "C" int sb_rope_norm_bwd(const void* x, void* d, const int* pos, const float* cos_sin, const void* q_nw, const void* k_nw, float* part,
+                                float* dw, int T, int Hq, int Hkv, int D, int x_stride, int d_stride, int blocks, float eps, cudaStream_t s) {
+  if (blocks <= 0 || T <= 0 || !rope_vec(x, x_stride, q_nw, cos_sin) || !rope_vec(d, d_stride, k_nw, cos_sin) || q_nw == nullptr || k_nw == nullptr)
     return (int)cudaErrorInvalidValue;
+#define SB_RNB(DV)                                                                                                                  \
+  if (D == DV)                                                                                                                      \
+    sb::rope_norm_bwd_kernel<DV><<<blocks, 256, 0, s>>>((const bf16*)x, (bf16*)d, pos, cos_sin, (const bf16*)q_nw, (const bf16*)k_nw, part, T, \
+                                                        Hq, Hkv, x_stride, d_stride, eps);
+  SB_RNB(64) else SB_RNB(128) else return (int)cudaErrorInvalidValue;
+#undef SB_RNB
+  sb::rmsnorm_dw_reduce_kernel<<<sb::dw_reduce_blocks(2 * D), sb::DW_THREADS, 0, s>>>(part, dw, blocks, 2 * D, 0);
   return (int)cudaGetLastError();
 }
 
@@ -525,14 +719,14 @@ extern "C" int sb_rope_kv_write(void* qkv, const int* pos, const float* cos_sin,
                                 float eps, cudaStream_t s) {
   if (T == 0) return 0;
   if ((row_stride & 1) || (reinterpret_cast<uintptr_t>(qkv) & 3)) return (int)cudaErrorInvalidValue;
-  const long warps = (long)T * (Hq + 2 * Hkv);
-  const int blocks = (int)((warps * 32 + 127) / 128);
-#define SB_RKW(DV)                                                                                                     \
-  if (D == DV)                                                                                                         \
-    return (int)sb::launch_pdl(sb::rope_kv_write_kernel<DV>, dim3(blocks), dim3(128), 0, s, (bf16*)qkv, pos, cos_sin,  \
-                               (const bf16*)q_nw, (const bf16*)k_nw, slots, (bf16*)k_cache, (bf16*)v_cache, T, Hq, Hkv, \
-                               row_stride, eps);
-  SB_RKW(64) SB_RKW(128) SB_RKW(256)
+  // a warp has heads of both kinds: both are normed or neither
+  const bool vec = (q_nw == nullptr) == (k_nw == nullptr) && rope_vec(qkv, row_stride, q_nw, cos_sin) && rope_vec(k_cache, 0, k_nw, nullptr) && rope_vec(v_cache, 0, nullptr, nullptr);
+#define SB_RKW(DV, V)                                                                                                       \
+  if (D == DV && vec == V)                                                                                                  \
+    return (int)sb::launch_pdl(sb::rope_kv_write_kernel<DV, V>, dim3(rope_blocks((long)T * (Hq + 2 * Hkv), V ? DV / 16 : 32)), dim3(128), 0, s, \
+                               (bf16*)qkv, pos, cos_sin, (const bf16*)q_nw, (const bf16*)k_nw, slots, (bf16*)k_cache, (bf16*)v_cache, T, Hq, \
+                               Hkv, row_stride, eps);
+  SB_RKW(64, true) SB_RKW(64, false) SB_RKW(128, true) SB_RKW(128, false) SB_RKW(256, true) SB_RKW(256, false)
 #undef SB_RKW
   return (int)cudaErrorInvalidValue;
 }

@@ -451,6 +451,38 @@ def _head_norm_bwd(x, dy, w, eps):
     return dx, dw.to(w.dtype)
 
 
+def rope_norm_bwd_(qkv, dqkv, positions, cos_sin, q_norm_w, k_norm_w, Hq, Hkv, D, eps):
+    """Backward of per-head RMSNorm and rotation of packed rows: the q and k gradients in ``dqkv`` become those of ``qkv`` in place.
+    Returns the gradients of the two weights (None where they went to ``main_grad``)."""
+    T = qkv.shape[0]
+    if all(t.data_ptr() % 16 == 0 for t in (qkv, dqkv, cos_sin)) and qkv.stride(0) % 8 == 0 and dqkv.stride(0) % 8 == 0 and T:
+        blocks = min(4 * _lib.sm_count(qkv.device), -(-T * Hq * D // 4096))
+        part = torch.empty(blocks, 2, D, dtype=torch.float32, device=qkv.device)
+        dw = torch.empty(2, D, dtype=torch.float32, device=qkv.device)
+        qw, kw = (w if w.data_ptr() % 16 == 0 else w.clone() for w in (q_norm_w, k_norm_w))
+        rc = _lib.lib().sb_rope_norm_bwd(P(qkv), P(dqkv), P(positions), P(cos_sin), P(qw), P(kw), P(part), P(dw), T, Hq, Hkv, D,
+                                         qkv.stride(0), dqkv.stride(0), blocks, float(eps), _lib.stream())  # fmt: skip
+        _lib.check(rc, "sb_rope_norm_bwd")
+        return tuple(_norm_weight_grad(w, g) for w, g in zip((q_norm_w, k_norm_w), dw))
+    _rope_launch(dqkv, dqkv, positions, cos_sin, None, None, Hq + Hkv, 0, D, eps, -1.0)  # inverse rotation, in place
+    x3, d3 = (t.view(T, Hq + 2 * Hkv, D) for t in (qkv, dqkv))
+    dq, dqw = _head_norm_bwd(x3[:, :Hq], d3[:, :Hq], q_norm_w, eps)
+    dk, dkw = _head_norm_bwd(x3[:, Hq : Hq + Hkv], d3[:, Hq : Hq + Hkv], k_norm_w, eps)
+    d3[:, :Hq].copy_(dq)
+    d3[:, Hq : Hq + Hkv].copy_(dk)
+    return dqw, dkw
+
+
+def _norm_weight_grad(w, dw):
+    """fp32 gradient of a norm's weight: added to its ``main_grad`` (then None), or in the weight's type."""
+    main_grad = getattr(w, "main_grad", None)
+    if main_grad is None:
+        return dw.to(w.dtype)
+    main_grad.add_(dw)
+    w.grad_added_to_main_grad = True
+    return None
+
+
 def rope_qk(qkv, positions, cos_sin, Hq, Hkv, D, q_norm_w=None, k_norm_w=None, eps=1e-6):
     return _RopeQK.apply(qkv, positions, cos_sin, q_norm_w, k_norm_w, Hq, Hkv, D, eps)
 

@@ -243,7 +243,7 @@ class _RopeAttentionCUDA(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        from slime_b200.ops import _head_norm_bwd, _rope_launch
+        from slime_b200.ops import _rope_launch, rope_norm_bwd_
 
         qkv, rot, out, lse, seg, positions, cos_sin, q_norm_w, k_norm_w = ctx.saved_tensors
         Hq, Hkv, D, eps, scale = ctx.dims
@@ -255,13 +255,11 @@ class _RopeAttentionCUDA(torch.autograd.Function):
         d3 = dqkv.view(T, Hq + 2 * Hkv, D)
         flash_bwd(r3[:, :Hq], r3[:, Hq : Hq + Hkv], x3[:, Hq + Hkv :], out, dout.reshape(T, Hq, D), lse, seg, scale,
                   dq=d3[:, :Hq], dk=d3[:, Hq : Hq + Hkv], dv=d3[:, Hq + Hkv :])  # fmt: skip
-        _rope_launch(dqkv, dqkv, positions, cos_sin, None, None, Hq + Hkv, 0, D, eps, -1.0)  # inverse rotation, in place
         dqw = dkw = None
         if has_norm:
-            dq, dqw = _head_norm_bwd(x3[:, :Hq], d3[:, :Hq], q_norm_w, eps)
-            dk, dkw = _head_norm_bwd(x3[:, Hq : Hq + Hkv], d3[:, Hq : Hq + Hkv], k_norm_w, eps)
-            d3[:, :Hq].copy_(dq)
-            d3[:, Hq : Hq + Hkv].copy_(dk)
+            dqw, dkw = rope_norm_bwd_(qkv, dqkv, positions, cos_sin, q_norm_w, k_norm_w, Hq, Hkv, D, eps)
+        else:
+            _rope_launch(dqkv, dqkv, positions, cos_sin, None, None, Hq + Hkv, 0, D, eps, -1.0)  # inverse rotation, in place
         return dqkv, None, None, dqw, dkw, None, None, None, None, None, None
 
 
