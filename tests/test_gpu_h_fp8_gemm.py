@@ -135,3 +135,25 @@ def test_fp8_engine_on_gpu_tracks_the_bf16_engine(kernels):
     assert float(np.median(diffs)) < 0.15 and float(np.mean(diffs)) < 0.35, (float(np.median(diffs)), float(np.mean(diffs)))
     for e in engines.values():
         e.shutdown()
+
+
+@pytest.mark.parametrize("M,K", [(1, 128), (3, 384), (777, 9728), (4000, 128)])
+@pytest.mark.parametrize("pow2", [0, 1])
+def test_activation_quant_in_16_byte_pieces(kernels, M, K, pow2):
+    """Rows of whole 16-byte pieces and rows that are not take different kernels: the same bits, also for zeros, infinities and NaN."""
+    from slime_b200.ops import _lib
+
+    torch.manual_seed(M)
+    wide = torch.randn(M, K + 4, device="cuda").bfloat16()
+    wide[0, :128] = 0
+    if K > 128:
+        wide[0, 130], wide[-1, 260] = float("inf"), float("nan")
+    got = []
+    for x in (wide[:, :K].contiguous(), wide[:, :K]):
+        q = torch.empty(M, K, dtype=torch.uint8, device="cuda")
+        s, st = torch.empty(M, K // 128, device="cuda"), torch.empty(K // 128, M, device="cuda")
+        rc = _lib.lib().sb_group_fp8_quant_1x128(x.data_ptr(), q.data_ptr(), s.data_ptr(), st.data_ptr(), M, K, x.stride(0), K, pow2, _lib.stream())
+        _lib.check(rc, "sb_group_fp8_quant_1x128")
+        got.append((q, s.view(torch.int32), st.view(torch.int32)))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
