@@ -39,42 +39,60 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 
+// Sum over the block, one barrier: `scratch` is two rows of 32 that are used in turn (a thread may be one call ahead of the others).
+__device__ __forceinline__ float block_sum_turn(float v, float (&scratch)[2][32], int turn) {
+  v = warp_sum(v);
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) scratch[turn][threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(lane < static_cast<int>(blockDim.x >> 5) ? scratch[turn][lane] : 0.f);
+}
+
 // y = rmsnorm(x (+ res)) * w ; optionally res_out = x + res (bf16) ; rstd[T] saved for backward.
-// H % 8 == 0, H <= 8192. grid = T rows. XT = bf16, or float when x is the fp32 sum left by a split-K projection.
+// H % 8 == 0, H <= 8192. XT = bf16, or float when x is the fp32 sum left by a split-K projection. Bound by HBM: rows of up to 1024 elements
+// have a warp each (four vectors a lane, all loads first, no barrier), wider ones a block with one vector a thread. Blocks of 256 threads
+// for every row left half of them idle at 896 elements: 15800 rows 39 -> 20 us.
 template <typename XT>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                   __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H, float eps) {
-  __shared__ float scratch[32];
+rmsnorm_fwd_warp_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
+                        __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int T, int H, float eps) {
+  constexpr int VPL = 4;
   pdl_wait();  // inputs come from the previous kernel in the stream
   pdl_launch_dependents();
-  const size_t row = blockIdx.x;
-  const int nvec = H >> 3;
-  float v[NORM_MAX_VEC][8];
-  float ss = 0.f;
+  const int nvec = H >> 3, lane = threadIdx.x & 31;
+  const size_t row = static_cast<size_t>(blockIdx.x) * (NORM_THREADS / 32) + (threadIdx.x >> 5);
+  if (row >= static_cast<size_t>(T)) return;
+  float v[VPL][8];
+  uint4 r[VPL];
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_VEC; ++j) {
-    const int c = threadIdx.x + j * NORM_THREADS;
+  for (int j = 0; j < VPL; ++j) {
+    const int c = lane + 32 * j;
+    r[j] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[j][i] = 0.f;
     if (c < nvec) {
       load8(x + row * H + c * 8, v[j]);
-      if (res != nullptr) {
-        float r[8];
-        load8(res + row * H + c * 8, r);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[j][i] += r[i];
-      }
-      if (res_out != nullptr) store8(res_out + row * H + c * 8, v[j]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) ss += v[j][i] * v[j][i];
+      if (res != nullptr) r[j] = *reinterpret_cast<const uint4*>(res + row * H + c * 8);
     }
   }
-  ss = block_sum<NORM_THREADS>(ss, scratch);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
+  float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < NORM_MAX_VEC; ++j) {
-    const int c = threadIdx.x + j * NORM_THREADS;
+  for (int j = 0; j < VPL; ++j) {
+    const int c = lane + 32 * j;
+    float f[8];
+    unpack8(r[j], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[j][i] += f[i];
+      ss += v[j][i] * v[j][i];
+    }
+    if (res_out != nullptr && c < nvec) store8(res_out + row * H + c * 8, v[j]);
+  }
+  const float rstd = rsqrtf(warp_sum(ss) / H + eps);
+  if (lane == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
+#pragma unroll
+  for (int j = 0; j < VPL; ++j) {
+    const int c = lane + 32 * j;
     if (c < nvec) {
       float g[8], o[8];
       load8(w + c * 8, g);
@@ -85,72 +103,100 @@ rmsnorm_fwd_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ r
   }
 }
 
+template <typename XT>
+__global__ void __launch_bounds__(1024)
+rmsnorm_fwd_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
+                   __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H, float eps) {
+  __shared__ float scratch[2][32];
+  pdl_wait();
+  pdl_launch_dependents();
+  const size_t at = static_cast<size_t>(blockIdx.x) * H + threadIdx.x * 8;
+  const bool in = static_cast<int>(threadIdx.x) < (H >> 3);
+  float v[8] = {}, g[8] = {};
+  float ss = 0.f;
+  if (in) {
+    load8(x + at, v);
+    load8(w + threadIdx.x * 8, g);
+    if (res != nullptr) {
+      float r[8];
+      load8(res + at, r);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] += r[i];
+    }
+    if (res_out != nullptr) store8(res_out + at, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+  }
+  const float rstd = rsqrtf(block_sum_turn(ss, scratch, 0) / H + eps);
+  if (threadIdx.x == 0 && rstd_out != nullptr) rstd_out[blockIdx.x] = rstd;
+  if (!in) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = v[i] * rstd * g[i];
+  store8(y + at, v);
+}
+
+template <typename XT>
+static cudaError_t launch_rmsnorm_fwd(const XT* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* res_out,
+                                      float* rstd, int T, int H, float eps, cudaStream_t s) {
+  if (H <= 1024)
+    return launch_pdl(rmsnorm_fwd_warp_kernel<XT>, dim3((T + NORM_THREADS / 32 - 1) / (NORM_THREADS / 32)), dim3(NORM_THREADS), 0, s, x, res, w, y,
+                      res_out, rstd, T, H, eps);
+  return launch_pdl(rmsnorm_fwd_kernel<XT>, dim3(T), dim3(((H >> 3) + 31) / 32 * 32), 0, s, x, res, w, y, res_out, rstd, H, eps);
+}
+
 // Backward of y = rmsnorm(h) * w for a strip of rows per CTA (h = the summed residual input).
 //   dh = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ dres_in)
 //   dw_partial[cta, :] = sum over the CTA's rows of dy * xhat
 // dw_partial is scratch of shape [gridDim.x, H] fp32, reduced by rmsnorm_dw_reduce_kernel.
-__global__ void __launch_bounds__(NORM_THREADS)
+// One vector a thread, the next row's loads in flight while this row's sum goes round, one barrier a row: bound by HBM. Up to four
+// vectors a thread, loads and three barriers in turn, took 200 us for 9198 rows of 2560, this 46.
+__global__ void __launch_bounds__(1024)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dh,
                    float* __restrict__ dw_partial, int T, int H) {
-  __shared__ float scratch[32];
-  const int nvec = H >> 3;
-  float dwacc[NORM_MAX_VEC][8];
-  float g[NORM_MAX_VEC][8];
-#pragma unroll
-  for (int j = 0; j < NORM_MAX_VEC; ++j) {
-    const int c = threadIdx.x + j * NORM_THREADS;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dwacc[j][i] = 0.f;
-    if (c < nvec) load8(w + c * 8, g[j]);
-  }
-  for (size_t row = blockIdx.x; row < static_cast<size_t>(T); row += gridDim.x) {
-    const float rs = rstd[row];
-    float xh[NORM_MAX_VEC][8], dyw[NORM_MAX_VEC][8];
+  __shared__ float scratch[2][32];
+  const int c = threadIdx.x * 8;
+  const bool in = c < H;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  float dwacc[8] = {}, g[8] = {};
+  if (in) load8(w + c, g);
+  uint4 na = none, nb = none, nr = none;
+  float nrs = 0.f;
+  auto fetch = [&](size_t row) {
+    if (row >= static_cast<size_t>(T)) return;
+    nrs = rstd[row];
+    if (!in) return;
+    na = *reinterpret_cast<const uint4*>(dy + row * H + c);
+    nb = *reinterpret_cast<const uint4*>(h + row * H + c);
+    if (dres_in != nullptr) nr = *reinterpret_cast<const uint4*>(dres_in + row * H + c);
+  };
+  fetch(blockIdx.x);
+  int turn = 0;
+  for (size_t row = blockIdx.x; row < static_cast<size_t>(T); row += gridDim.x, turn ^= 1) {
+    const float rs = nrs;
+    float a[8], xh[8], r[8];
+    unpack8(na, a);
+    unpack8(nb, xh);
+    unpack8(nr, r);
+    fetch(row + gridDim.x);
     float dot = 0.f;
 #pragma unroll
-    for (int j = 0; j < NORM_MAX_VEC; ++j) {
-      const int c = threadIdx.x + j * NORM_THREADS;
-      if (c < nvec) {
-        float a[8], b[8];
-        load8(dy + row * H + c * 8, a);
-        load8(h + row * H + c * 8, b);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          xh[j][i] = b[i] * rs;
-          dwacc[j][i] += a[i] * xh[j][i];
-          dyw[j][i] = a[i] * g[j][i];
-          dot += dyw[j][i] * xh[j][i];
-        }
-      }
+    for (int i = 0; i < 8; ++i) {
+      xh[i] *= rs;
+      dwacc[i] += a[i] * xh[i];
+      a[i] *= g[i];
+      dot += a[i] * xh[i];
     }
-    dot = block_sum<NORM_THREADS>(dot, scratch) / H;
+    dot = block_sum_turn(dot, scratch, turn) / H;
 #pragma unroll
-    for (int j = 0; j < NORM_MAX_VEC; ++j) {
-      const int c = threadIdx.x + j * NORM_THREADS;
-      if (c < nvec) {
-        float o[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rs * (dyw[j][i] - xh[j][i] * dot);
-        if (dres_in != nullptr) {
-          float r[8];
-          load8(dres_in + row * H + c * 8, r);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] += r[i];
-        }
-        store8(dh + row * H + c * 8, o);
-      }
-    }
+    for (int i = 0; i < 8; ++i) a[i] = rs * (a[i] - xh[i] * dot) + r[i];
+    if (in) store8(dh + row * H + c, a);
   }
-#pragma unroll
-  for (int j = 0; j < NORM_MAX_VEC; ++j) {
-    const int c = threadIdx.x + j * NORM_THREADS;
-    if (c < nvec) {
-      float4* dst = reinterpret_cast<float4*>(dw_partial + static_cast<size_t>(blockIdx.x) * H + c * 8);
-      dst[0] = make_float4(dwacc[j][0], dwacc[j][1], dwacc[j][2], dwacc[j][3]);
-      dst[1] = make_float4(dwacc[j][4], dwacc[j][5], dwacc[j][6], dwacc[j][7]);
-    }
+  if (in) {
+    float4* dst = reinterpret_cast<float4*>(dw_partial + static_cast<size_t>(blockIdx.x) * H + c);
+    dst[0] = make_float4(dwacc[0], dwacc[1], dwacc[2], dwacc[3]);
+    dst[1] = make_float4(dwacc[4], dwacc[5], dwacc[6], dwacc[7]);
   }
 }
 
@@ -175,7 +221,7 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw,
 }
 
 // Same backward for rows of at most 1024 elements: one WARP per row, so a row costs one shuffle reduction and no
-// block barrier, and every warp keeps 2 * VPL independent 16-byte loads in flight. Lane l owns the 8-element
+// block barrier, and every warp keeps 3 * VPL independent 16-byte loads in flight. Lane l owns the 8-element
 // vectors l, l + 32, ... (VPL of them). The per-column dw sums of the CTA's 8 warps are combined in shared memory in
 // warp order (deterministic) and written as one partial row per CTA.
 template <int VPL>
@@ -200,12 +246,13 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
   for (size_t row = static_cast<size_t>(blockIdx.x) * WARPS + warp; row < static_cast<size_t>(T);
        row += static_cast<size_t>(gridDim.x) * WARPS) {
     const float rs = rstd[row];
-    uint4 ra[VPL], rb[VPL];
+    uint4 ra[VPL], rb[VPL], rr[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {  // all loads of the row first
       const int c = lane + 32 * j;
-      ra[j] = rb[j] = make_uint4(0, 0, 0, 0);
+      ra[j] = rb[j] = rr[j] = make_uint4(0, 0, 0, 0);
       if (c < nvec) {
+        if (dres_in != nullptr) rr[j] = *reinterpret_cast<const uint4*>(dres_in + row * H + c * 8);
         ra[j] = *reinterpret_cast<const uint4*>(dy + row * H + c * 8);
         rb[j] = *reinterpret_cast<const uint4*>(h + row * H + c * 8);
       }
@@ -232,7 +279,7 @@ rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
         float a[8], b[8], r[8], g[8], o[8];
         unpack8(ra[j], a);
         unpack8(rb[j], b);
-        unpack8(dres_in != nullptr ? *reinterpret_cast<const uint4*>(dres_in + row * H + c * 8) : make_uint4(0, 0, 0, 0), r);
+        unpack8(rr[j], r);
         unpack8(gw[j], g);
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = rs * (a[i] * g[i] - b[i] * rs * dot) + r[i];
@@ -269,7 +316,7 @@ static cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat
   else if (nvec <= 128)
     rmsnorm_bwd_warp_kernel<4><<<num_ctas, NORM_THREADS, 0, s>>>(dy, h, w, rstd, dres_in, dh, dw_partial, T, H);
   else
-    rmsnorm_bwd_kernel<<<num_ctas, NORM_THREADS, 0, s>>>(dy, h, w, rstd, dres_in, dh, dw_partial, T, H);
+    rmsnorm_bwd_kernel<<<num_ctas, (nvec + 31) / 32 * 32, 0, s>>>(dy, h, w, rstd, dres_in, dh, dw_partial, T, H);
   rmsnorm_dw_reduce_kernel<<<dw_reduce_blocks(H), DW_THREADS, 0, s>>>(dw_partial, dw, num_ctas, H, accumulate_dw);
   return cudaGetLastError();
 }
@@ -655,8 +702,7 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
                               int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
   if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8) return (int)cudaErrorInvalidValue;
-  return (int)sb::launch_pdl(sb::rmsnorm_fwd_kernel<bf16>, dim3(T), dim3(sb::NORM_THREADS), 0, s, (const bf16*)x,
-                             (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, H, eps);
+  return (int)sb::launch_rmsnorm_fwd((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
 // Same, with x in fp32 (res, w, y, res_out stay bf16).
@@ -664,8 +710,7 @@ extern "C" int sb_rmsnorm_fwd_f32x(const float* x, const void* res, const void* 
                                    int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
   if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8) return (int)cudaErrorInvalidValue;
-  return (int)sb::launch_pdl(sb::rmsnorm_fwd_kernel<float>, dim3(T), dim3(sb::NORM_THREADS), 0, s, x, (const bf16*)res,
-                             (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, H, eps);
+  return (int)sb::launch_rmsnorm_fwd(x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
 // dw_partial: scratch [num_ctas, H] fp32 supplied by the caller; dw: [H] fp32.

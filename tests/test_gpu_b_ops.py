@@ -320,3 +320,32 @@ def test_rope_kv_write_matches_separate_ops(kernels, Hq, Hkv, D, norm):
     unused = torch.ones(slots_n, dtype=torch.bool, device="cuda")
     unused[slots[ok].long()] = False
     assert (kc[unused] == 0).all() and (vc[unused] == 0).all()
+
+
+@pytest.mark.parametrize("T,H", [(1, 8), (9, 264), (8, 1024), (7, 1032), (300, 2560), (5, 8192)])
+@pytest.mark.parametrize("fp32_in,res", [(False, False), (False, True), (True, True)])
+def test_rmsnorm_at_the_edges_of_its_forms(kernels, T, H, fp32_in, res):
+    """A warp per row up to 1024 elements, a block per row above: against 64 bits, bf16 results with one rounding; gradients of the weight
+    are fp32 sums over the rows."""
+    from slime_b200 import ops
+
+    torch.manual_seed(H)
+    x = torch.randn(T, H, device="cuda").to(torch.float32 if fp32_in else torch.bfloat16)
+    r = torch.randn(T, H, device="cuda").bfloat16() if res else None
+    w = (torch.rand(H, device="cuda") + 0.5).bfloat16().requires_grad_()
+    if not fp32_in:
+        x.requires_grad_()
+    y, h = ops.rmsnorm(x, w, 1e-6, r)
+    s = x.detach().double() + (r.double() if res else 0)
+    want = s * torch.rsqrt(s.square().mean(-1, keepdim=True) + 1e-6) * w.detach().double()
+    torch.testing.assert_close(y.double(), want, rtol=2**-8, atol=1e-5)
+    torch.testing.assert_close(h.double(), s, rtol=2**-8, atol=1e-5)
+    if fp32_in:
+        return
+    dy, dh = torch.randn_like(y), torch.randn_like(h)
+    hs = h.detach().double().requires_grad_()  # the kernel differentiates at the rounded sum
+    w64 = w.detach().double().requires_grad_()
+    (hs * torch.rsqrt(hs.square().mean(-1, keepdim=True) + 1e-6) * w64).backward(dy.double())
+    torch.autograd.backward([y, h], [dy, dh])
+    torch.testing.assert_close(x.grad.double(), hs.grad + dh.double(), rtol=2**-7, atol=2**-6)
+    torch.testing.assert_close(w.grad.double(), w64.grad, rtol=2**-7, atol=1e-3 * T**0.5)
