@@ -108,6 +108,8 @@ def _pick_pair(M: int, N: int, K: int, split_last: bool, sms: int = 148) -> int:
     best, width = 1e30, 0
     for bn, rate in ((256, 1.0), (224, 0.92), (192, 0.85), (128, 0.65)):
         tiles = -(-M // 256) * -(-N // bn)
+        if tiles < pairs // 2 and not split_last:  # one tile's chain of k-blocks bounds the call: smaller tiles on single SMs, or slices of K
+            continue
         if split_last and tiles >= pairs:  # with fewer tiles the uniform slices of the one-SM kernel are faster (35 and 39 us: 896 x 896 x 15800)
             waves = tiles / pairs
         elif split_last:
@@ -166,6 +168,13 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
         res = _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms) if width else None
         if res is not None:
             return res
+    if out_dtype == torch.bfloat16 and bn is None and splitk is None and K >= 16384 and N % 4 == 0 and not accumulate:
+        # a bf16 output of few tiles over a very long K (gradients of few rows behind a head): sums of K slices in fp32, then rounded.
+        # 265 x 896 x 151936: 661 -> 120 us, 100 x 2560 x 16384: 80 -> 34. The fill and the conversion cost about 5.
+        slices = _pick_splitk(M, N, K, 128, _lib.sm_count(a.device))
+        if slices > 1:
+            res = gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, out_dtype=torch.float32, bn=128, splitk=slices)
+            return res.to(out_dtype) if out is None else out.copy_(res)
     bn = bn or _pick_bn(M, N)
     can_split = out_dtype == torch.float32 and (accumulate or (out is None and N % 4 == 0))  # TMA reduce-add: 16-byte rows
     if splitk is None:
@@ -239,7 +248,7 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
         ctx.save_for_backward(x, weight)
-        ctx.has_bias = bias is not None
+        ctx.has_bias, ctx.bias = bias is not None, bias
         x2 = x.reshape(-1, x.shape[-1])
         y = gemm(x2, weight, bias=bias)
         return y.view(*x.shape[:-1], weight.shape[0])
@@ -263,8 +272,24 @@ class _Linear(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0).to(dy.dtype)
+            db = _bias_grad(dy2, ctx.bias)
         return dx, dw, db
+
+
+def _bias_grad(dy, bias):
+    """Column sums of ``dy`` [T, N]: into the bias's fp32 ``main_grad`` (then None), or returned."""
+    T, N = dy.shape
+    if not dy.is_cuda or dy.dtype != torch.bfloat16 or T == 0 or N % 8 or dy.stride(0) % 8 or dy.data_ptr() % 16:
+        return dy.float().sum(0).to(dy.dtype)
+    main_grad = getattr(bias, "main_grad", None)
+    direct = main_grad is not None and main_grad.dtype == torch.float32 and main_grad.is_contiguous()
+    part = torch.empty(min(64, -(-T // 8)), N, dtype=torch.float32, device=dy.device)
+    out = main_grad if direct else torch.empty(N, dtype=torch.float32, device=dy.device)
+    _lib.check(_lib.lib().sb_column_sum(P(dy), P(part), P(out), T, N, dy.stride(0), int(direct), _lib.stream()), "sb_column_sum")
+    if not direct:
+        return out.to(dy.dtype)
+    bias.grad_added_to_main_grad = True
+    return None
 
 
 def linear(x, weight, bias=None):
@@ -327,13 +352,16 @@ class _RMSNorm(torch.autograd.Function):
             dh = torch.empty_like(h)
             n = min(_norm_ctas(dy.device), max(T, 1))
             part = torch.empty(n, H, dtype=torch.float32, device=dy.device)
-            dw = torch.empty(H, dtype=torch.float32, device=dy.device)
-            rc = _lib.lib().sb_rmsnorm_bwd(P(dy2), P(h), P(weight), P(rstd), P(dres), P(dh), P(part), P(dw), T, H, n, 0,
+            held = getattr(weight, "main_grad", None)
+            direct = held is not None and held.dtype == torch.float32 and held.is_contiguous() and T > 0
+            dw = held if direct else torch.empty(H, dtype=torch.float32, device=dy.device)
+            rc = _lib.lib().sb_rmsnorm_bwd(P(dy2), P(h), P(weight), P(rstd), P(dres), P(dh), P(part), P(dw), T, H, n, int(direct),
                                            _lib.stream())
             _lib.check(rc, "sb_rmsnorm_bwd")
         main_grad = getattr(weight, "main_grad", None)
         if main_grad is not None:
-            main_grad.add_(dw)
+            if dw is not main_grad:
+                main_grad.add_(dw)
             weight.grad_added_to_main_grad = True
             dw_out = None
         else:

@@ -79,6 +79,7 @@ _SIGS = {
     "sb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_fwd_f32x": [P, P, P, P, P, P, I, I, F, P],
     "sb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, I, I, I, I, P],
+    "sb_column_sum": [P, P, P, I, I, L, I, P],
     "sb_rope_norm_bwd": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P],
     "sb_rope": [P, P, P, P, P, P, I, I, I, I, I, I, F, F, P],
     "sb_swiglu_fwd": [P, P, L, I, P, P],

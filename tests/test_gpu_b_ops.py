@@ -349,3 +349,34 @@ def test_rmsnorm_at_the_edges_of_its_forms(kernels, T, H, fp32_in, res):
     torch.autograd.backward([y, h], [dy, dh])
     torch.testing.assert_close(x.grad.double(), hs.grad + dh.double(), rtol=2**-7, atol=2**-6)
     torch.testing.assert_close(w.grad.double(), w64.grad, rtol=2**-7, atol=1e-3 * T**0.5)
+
+
+@pytest.mark.parametrize("T,N", [(1, 8), (7, 264), (8, 256), (513, 1000), (15800, 1152)])
+@pytest.mark.parametrize("held", [False, True])
+def test_bias_gradient(kernels, T, N, held):
+    """Column sums in fp32: within the roundings of T additions of 64 bits; without ``main_grad`` rounded to bf16 once."""
+    from slime_b200 import ops
+
+    torch.manual_seed(T)
+    dy = torch.randn(T, N + 8, device="cuda").bfloat16()[:, :N]
+    bias = torch.zeros(N, device="cuda", dtype=torch.bfloat16)
+    want = dy.double().sum(0)
+    if held:
+        bias.main_grad = torch.ones(N, device="cuda")
+    got = ops._bias_grad(dy, bias)
+    assert (got is None) == held
+    torch.testing.assert_close((bias.main_grad - 1 if held else got).double(), want, rtol=1e-5 if held else 2**-8, atol=2e-6 * T**0.5 + 2e-7)
+
+
+@pytest.mark.parametrize("M,N,K", [(265, 896, 151936), (1, 8, 16384), (130, 136, 20000)])
+def test_few_rows_over_a_long_sum(kernels, M, N, K):
+    """A bf16 output summed from K slices in fp32: one rounding of sums whose terms come in another order."""
+    from slime_b200 import ops
+
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(K, N, device="cuda") * 0.02).bfloat16()
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(a, b, b_mn=True, out=out)
+    want = a.double() @ b.double()
+    for got in (out, ops.gemm(a, b, b_mn=True)):
+        torch.testing.assert_close(got.double(), want, rtol=2**-8, atol=1e-3)
