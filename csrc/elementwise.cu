@@ -48,9 +48,17 @@ __device__ __forceinline__ float block_sum_turn(float v, float (&scratch)[2][32]
   return warp_sum(lane < static_cast<int>(blockDim.x >> 5) ? scratch[turn][lane] : 0.f);
 }
 
+__device__ __forceinline__ float square_sum8(const float (&v)[8]) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s = fmaf(v[i], v[i], s);
+  return s;
+}
+
 // y = rmsnorm(x (+ res)) * w ; optionally res_out = x + res (bf16) ; rstd[T] saved for backward.
 // H % 8 == 0, H <= 8192. XT = bf16, or float when x is the fp32 sum left by a split-K projection. Bound by HBM: rows of up to 1024 elements
-// have a warp each (four vectors a lane, all loads first, no barrier), wider ones a block with one vector a thread. Blocks of 256 threads
+// have a warp each (four vectors a lane, all loads first, no barrier), wider ones, and the few rows of a decode step, whose time is that of
+// one row, a block with one vector a thread. Both add a row's squares up in the same order, so a row's bits don't depend on the others. Blocks of 256 threads
 // for every row left half of them idle at 896 elements: 15800 rows 39 -> 20 us.
 template <typename XT>
 __global__ void __launch_bounds__(NORM_THREADS)
@@ -75,20 +83,18 @@ rmsnorm_fwd_warp_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restric
       if (res != nullptr) r[j] = *reinterpret_cast<const uint4*>(res + row * H + c * 8);
     }
   }
-  float ss = 0.f;
+  float part[VPL];
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
     const int c = lane + 32 * j;
     float f[8];
     unpack8(r[j], f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[j][i] += f[i];
-      ss += v[j][i] * v[j][i];
-    }
+    for (int i = 0; i < 8; ++i) v[j][i] += f[i];
+    part[j] = warp_sum(square_sum8(v[j]));  // the sum that warp j of the block form has
     if (res_out != nullptr && c < nvec) store8(res_out + row * H + c * 8, v[j]);
   }
-  const float rstd = rsqrtf(warp_sum(ss) / H + eps);
+  const float rstd = rsqrtf(((part[0] + part[2]) + (part[1] + part[3])) / H + eps);  // as block_sum_turn pairs them
   if (lane == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
 #pragma unroll
   for (int j = 0; j < VPL; ++j) {
@@ -124,8 +130,7 @@ rmsnorm_fwd_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ r
       for (int i = 0; i < 8; ++i) v[i] += r[i];
     }
     if (res_out != nullptr) store8(res_out + at, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+    ss = square_sum8(v);
   }
   const float rstd = rsqrtf(block_sum_turn(ss, scratch, 0) / H + eps);
   if (threadIdx.x == 0 && rstd_out != nullptr) rstd_out[blockIdx.x] = rstd;
@@ -138,7 +143,7 @@ rmsnorm_fwd_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ r
 template <typename XT>
 static cudaError_t launch_rmsnorm_fwd(const XT* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y, __nv_bfloat16* res_out,
                                       float* rstd, int T, int H, float eps, cudaStream_t s) {
-  if (H <= 1024)
+  if (H <= 1024 && T >= 1024)
     return launch_pdl(rmsnorm_fwd_warp_kernel<XT>, dim3((T + NORM_THREADS / 32 - 1) / (NORM_THREADS / 32)), dim3(NORM_THREADS), 0, s, x, res, w, y,
                       res_out, rstd, T, H, eps);
   return launch_pdl(rmsnorm_fwd_kernel<XT>, dim3(T), dim3(((H >> 3) + 31) / 32 * 32), 0, s, x, res, w, y, res_out, rstd, H, eps);

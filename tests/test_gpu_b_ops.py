@@ -322,7 +322,7 @@ def test_rope_kv_write_matches_separate_ops(kernels, Hq, Hkv, D, norm):
     assert (kc[unused] == 0).all() and (vc[unused] == 0).all()
 
 
-@pytest.mark.parametrize("T,H", [(1, 8), (9, 264), (8, 1024), (7, 1032), (300, 2560), (5, 8192)])
+@pytest.mark.parametrize("T,H", [(1, 8), (9, 264), (8, 1024), (1025, 1024), (7, 1032), (300, 2560), (5, 8192)])
 @pytest.mark.parametrize("fp32_in,res", [(False, False), (False, True), (True, True)])
 def test_rmsnorm_at_the_edges_of_its_forms(kernels, T, H, fp32_in, res):
     """A warp per row up to 1024 elements, a block per row above: against 64 bits, bf16 results with one rounding; gradients of the weight
@@ -380,3 +380,15 @@ def test_few_rows_over_a_long_sum(kernels, M, N, K):
     want = a.double() @ b.double()
     for got in (out, ops.gemm(a, b, b_mn=True)):
         torch.testing.assert_close(got.double(), want, rtol=2**-8, atol=1e-3)
+
+
+@pytest.mark.parametrize("H", [8, 264, 520, 896, 1024])
+def test_norm_of_a_row_does_not_depend_on_the_number_of_rows(kernels, H):
+    """Few rows have a block each, many a warp: the same bits."""
+    from slime_b200 import ops
+
+    torch.manual_seed(H)
+    x, r, w = torch.randn(3000, H, device="cuda"), torch.randn(3000, H, device="cuda").bfloat16(), torch.rand(H, device="cuda").bfloat16()
+    for t in (x, x.bfloat16()):
+        many, few = ops.rmsnorm(t, w, 1e-6, r), ops.rmsnorm(t[:50], w, 1e-6, r[:50])
+        assert all(torch.equal(a[:50], b) for a, b in zip(many, few))
