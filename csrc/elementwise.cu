@@ -733,10 +733,16 @@ __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_
 
 using bf16 = __nv_bfloat16;
 
+// The norm kernels move 16 bytes at a time: what does not start on such a boundary is refused (on the device it is a misaligned address).
+static inline bool norm_aligned(const void* a, const void* b, const void* c, const void* d, const void* e) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d) |
+           reinterpret_cast<uintptr_t>(e)) & 15) == 0;
+}
+
 extern "C" int sb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                               int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_fwd((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
@@ -744,7 +750,7 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
 extern "C" int sb_rmsnorm_fwd_f32x(const float* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                                    int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_fwd(x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
@@ -753,7 +759,7 @@ extern "C" int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
                               void* dh, float* dw_partial, float* dw, int T, int H, int num_ctas, int accumulate_dw,
                               cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(dy, h, w, dres_in, dh)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_bwd((const bf16*)dy, (const bf16*)h, (const bf16*)w, rstd, (const bf16*)dres_in,
                                      (bf16*)dh, dw_partial, dw, T, H, num_ctas, accumulate_dw, s);
 }

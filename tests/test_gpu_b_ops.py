@@ -392,3 +392,14 @@ def test_norm_of_a_row_does_not_depend_on_the_number_of_rows(kernels, H):
     for t in (x, x.bfloat16()):
         many, few = ops.rmsnorm(t, w, 1e-6, r), ops.rmsnorm(t[:50], w, 1e-6, r[:50])
         assert all(torch.equal(a[:50], b) for a, b in zip(many, few))
+
+
+def test_norms_refuse_weights_off_a_16_byte_boundary(kernels):
+    """On the host, before anything is launched."""
+    from slime_b200 import ops
+
+    x, w = torch.randn(4, 64, device="cuda").bfloat16(), torch.ones(65, device="cuda", dtype=torch.bfloat16)[1:]
+    with pytest.raises(RuntimeError, match="sb_rmsnorm_fwd"):
+        ops.rmsnorm(x, w)
+    y, _ = ops.rmsnorm(x.requires_grad_(), torch.ones(64, device="cuda", dtype=torch.bfloat16))
+    assert torch.isfinite(y).all()
