@@ -90,7 +90,7 @@ def _pick_splitk(M: int, N: int, K: int, bn: int, sms: int = 148) -> int:
         return 1
     tiles = -(-M // 128) * -(-N // bn)
     kb = -(-K // 64)
-    if tiles * 2 > sms or kb < 16:
+    if tiles == 0 or tiles * 2 > sms or kb < 16:
         return 1
     return max(1, min(kb // 8, sms // tiles))
 
@@ -103,6 +103,8 @@ def _pick_pair(M: int, N: int, K: int, split_last: bool, sms: int = 148) -> int:
     tile 1.12 times as fast as one SM; narrower tiles reach 0.92 (224 wide), 0.85 (192) and 0.65 (128) of its rate per column, and pay
     where they fit N (896 = 4 x 224) or fill a wave. A pair's launch is about 2 us longer (two CTAs meet before and after), the
     time of 1900 columns of one k-block: 397 x 9728 x 896 takes 22.7 us on single SMs, 23.6 on pairs; 15800 x 9728 x 896 217 and 193."""
+    if M == 0 or N == 0 or K == 0:
+        return 0
     kb = -(-K // 64)
     pairs = sms // 2
     best, width = 1e30, 0
@@ -158,6 +160,8 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
         return gemm_simt(a, b, bias=bias, out=out, out_dtype=out_dtype)
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16, "sm_100a GEMM takes bf16 operands"
     assert out_dtype in (torch.bfloat16, torch.float32)
+    if M == 0 or N == 0 or K == 0:  # nothing to launch: an empty sum is zero (the weight gradient of no rows)
+        return _empty_product(bias, out, out_dtype, accumulate, M, N, a.device)
     if a.stride(-1) != 1:
         a = a.contiguous()
     if b.stride(-1) != 1:
@@ -197,6 +201,17 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_bf16")
     return out
+
+
+def _empty_product(bias, out, out_dtype, accumulate, M, N, device):
+    assert out is None or out.shape == (M, N)
+    assert not (accumulate and out_dtype != torch.float32), "accumulate needs an fp32 output"
+    if out is None:
+        assert not accumulate
+        out = torch.empty(M, N, dtype=out_dtype, device=device)
+    if not accumulate:
+        out.zero_()
+    return out if bias is None else out.add_(bias.to(out.dtype))
 
 
 def _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms):

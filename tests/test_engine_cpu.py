@@ -382,3 +382,12 @@ def test_deterministic_inference_switch_removes_batch_dependent_choices():
         assert alone.output_ids == crowd.output_ids and np.abs(np.array(alone.output_logprobs) - np.array(crowd.output_logprobs)).max() < 1e-5
     finally:
         ops.set_batch_invariant(False)
+
+
+def test_plans_of_empty_products():
+    """Whatever the other two sizes are, a product over nothing has no tiles to place and no k-blocks to cut."""
+    from slime_b200 import ops
+
+    for M, N, K in ((9728, 896, 0), (151936, 896, 0), (2560, 4096, 0), (0, 896, 151936), (0, 896, 896), (128, 0, 4096), (0, 0, 0)):
+        assert all(ops._pick_pair(M, N, K, cut) == 0 for cut in (False, True))
+        assert all(ops._pick_splitk(M, N, K, bn) == 1 for bn in (128, 256)) and ops.gemm_plan(M, N, K, True, 148)[2] == 1

@@ -104,3 +104,22 @@ def test_pairs_of_sms(kernels, M, N, K, a_mn, b_mn, width):
         ops._gemm_pair(a, b, a_mn, b_mn, None, acc, None, True, width, split, M, N, K, sms)
         torch.testing.assert_close(acc, one + 1.0, rtol=1e-5, atol=75 * 2.0**-24 * 4 * K**0.5)
     _lib.check_status("cuda")
+
+
+@pytest.mark.parametrize("out,inp", [(9728, 896), (2560, 4096), (64, 128)])
+def test_products_over_nothing(kernels, out, inp):
+    """No rows: a linear layer gives none, its input's gradient has none, its weights' gradients gain nothing, whatever the width."""
+    x = torch.empty(0, inp, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    for held in (True, False):
+        w = torch.randn(out, inp, device="cuda").bfloat16().requires_grad_()
+        b = torch.randn(out, device="cuda").bfloat16().requires_grad_()
+        if held:
+            w.main_grad = torch.ones(out, inp, device="cuda")
+        y = ops.linear(x, w, b)
+        y.backward(torch.empty_like(y))
+        assert y.shape == (0, out) and x.grad.shape == x.shape and (b.grad == 0).all()
+        assert (w.main_grad == 1).all() if held else (w.grad == 0).all()
+    a, c = torch.empty(0, 16384, device="cuda", dtype=torch.bfloat16), torch.randn(16384, 896, device="cuda").bfloat16()
+    assert ops.gemm(a, c, b_mn=True).shape == (0, 896)  # the gradient of no rows behind a head
+    empty, bias = torch.empty(5, 0, device="cuda", dtype=torch.bfloat16), torch.randn(7, device="cuda").bfloat16()
+    assert torch.equal(ops.gemm(empty, empty.new_empty(7, 0), bias=bias), bias.expand(5, 7))
