@@ -6,15 +6,18 @@
 // and bn / 2 rows of B; the tensor cores of both read both halves of B, so that a stage is 32 KB of shared memory for 128 x 256 outputs
 // per SM instead of 48 KB: a third less traffic from L2 and a third fewer operand reads, which is what bounds the one-SM kernel.
 //
-// Work: full waves of tiles first, one tile per pair and wave. Where the output is added to (ADD), the tiles of the last, partial
-// wave are cut along K into equal ranges over all pairs and summed by the TMA reduce-add that writes them anyway: a weight gradient
-// of 9728 x 896 is 152 tiles on 74 pairs and took three waves for work of 2.05.
+// Work: full waves of tiles first, one tile per pair and wave. Where the caller asks for it (outputs that are added to, and outputs of
+// less than a wave over a long K), the tiles of the last, partial wave are cut along K into as many slices as there are pairs for each: a weight
+// gradient of 9728 x 896 is 152 tiles on 74 pairs and took three waves for work of 2.05. A slice leaves its fp32 sums in a workspace,
+// and a second launch adds a tile's slices up in K order, so that the result is the same on every run. (Reduce-adds into
+// the output itself would save that launch, but they come in any order.)
 //
 // Grouped (weight gradients of experts): C is a stack of matrices, C[e] += A[rows of e]^T * B[rows of e], K = the rows of e.
 //
 // Bound by the tensor cores (and, in long runs, by the power limit). One SM per tile -> pairs, us: 9198 x 19456 x 2560 630 -> 573
-// (1598 TFLOP/s), 15800 x 9728 x 896 217 -> 193; weight gradients 9728 x 896 x 15800 318 -> 208, 2560 x 4096 x 9198 185 -> 134 (171 with
-// the last wave uncut). What is left below the peak is the last wave of outputs that are not added to, and K below 1000.
+// (1598 TFLOP/s), 15800 x 9728 x 896 217 -> 193; weight gradients 9728 x 896 x 15800 302 -> 211 (258 with
+// the last wave uncut), 2560 x 4096 x 9198 170 -> 133 (152). What is left below the peak is the last wave of outputs that are not added
+// to, and K below 1000.
 //
 // CTA = 6 warps as in gemm_sm100.cu: TMA producer, MMA issuer (leader CTA only), four epilogue warps.
 #include "common.cuh"
@@ -32,51 +35,74 @@ constexpr int GP_EPI = 4 * 2 * GP_EPI_BUF;
 constexpr int GP_SMEM = GP_STAGES * GP_STAGE + GP_EPI + (2 * GP_STAGES + 4) * 8 + 16 + 1024;
 constexpr int GP_PANEL = 16;  // row tiles of a panel: as many rows as in gemm_sm100.cu
 
+// One piece of work: a tile and a range of k-blocks.
+struct PairItem {
+  int m0, n0, z, kb0, kb1;  // kb absolute: rows of the group included
+  int part;                 // of a cut tile: where its sums go in the workspace; -1: a whole tile
+};
+
+// How the tiles behind the last full wave are cut: each of the `left` tiles into `slices` ranges of K, one a pair.
+struct PairCut {
+  int full, left, slices, pairs;
+};
+constexpr int GP_CUT_KB = 8;  // k-blocks of a slice at least: below, its way through the workspace takes longer than its products
+inline PairCut cut_last_wave(long long tiles, int num_kb, int num_sms, bool cut) {
+  PairCut c;
+  c.pairs = num_sms / 2;
+  c.full = static_cast<int>(tiles);
+  c.left = 0;
+  c.slices = 1;
+  const int rest = static_cast<int>(tiles % c.pairs);
+  if (cut && rest > 0) {
+    const int slices = c.pairs / rest < num_kb / GP_CUT_KB ? c.pairs / rest : num_kb / GP_CUT_KB;
+    if (slices > 1) {
+      c.full -= rest;
+      c.left = rest;
+      c.slices = slices;
+    }
+  }
+  const long long most = c.full > c.left * c.slices ? c.full : c.left * c.slices;
+  if (most < c.pairs) c.pairs = static_cast<int>(most);
+  return c;
+}
+
 struct PairShape {
   int M, N, K, bn;
   int groups;              // 1: plain
   const int* group_start;  // first row of A and B of group e (a multiple of 64)
   const int* group_rows;   // rows of group e; what follows them up to the next multiple of 64 is zero in A or B
-  int split_last;          // 1: cut the last wave along K
+  PairCut cut;
 };
 
-// One piece of work: a tile and a range of k-blocks.
-struct PairItem {
-  int m0, n0, z, kb0, kb1;  // kb absolute: rows of the group included
-};
+__device__ __forceinline__ void place_tile(const PairShape& s, int tiles_m, int tiles_n, int t, PairItem& it) {
+  const int per = tiles_m * tiles_n;
+  it.z = t / per;
+  t -= it.z * per;
+  const int per_panel = GP_PANEL * tiles_n;
+  const int panel = t / per_panel, r = t - panel * per_panel;
+  const int pm = min(GP_PANEL, tiles_m - panel * GP_PANEL);
+  it.m0 = (panel * GP_PANEL + r % pm) * 256;
+  it.n0 = (r / pm) * s.bn;
+}
 
 // The sequence of a pair's pieces; every role walks the same one.
 struct PairWalk {
-  int tiles_m, tiles_n, num_kb, tiles, full, pair, pairs;
-  long long lo, hi;  // k-blocks of the last wave that this pair takes
-  int tile;
+  int tiles_m, tiles_n, num_kb, tile, pair, pairs;
+  bool slice;  // one is still to come
   __device__ PairWalk(const PairShape& s, int pair_, int pairs_) {
     tiles_m = (s.M + 255) / 256;
     tiles_n = (s.N + s.bn - 1) / s.bn;
     num_kb = (s.K + GP_BK - 1) / GP_BK;
-    tiles = tiles_m * tiles_n * s.groups;
     pair = pair_;
     pairs = pairs_;
-    full = s.split_last ? tiles / pairs * pairs : tiles;
-    const long long left = static_cast<long long>(tiles - full) * num_kb;
-    lo = left * pair / pairs;
-    hi = left * (pair + 1) / pairs;
     tile = pair;
-  }
-  __device__ __forceinline__ void place(const PairShape& s, int t, PairItem& it) const {
-    const int per = tiles_m * tiles_n;
-    it.z = t / per;
-    t -= it.z * per;
-    const int per_panel = GP_PANEL * tiles_n;
-    const int panel = t / per_panel, r = t - panel * per_panel;
-    const int pm = min(GP_PANEL, tiles_m - panel * GP_PANEL);
-    it.m0 = (panel * GP_PANEL + r % pm) * 256;
-    it.n0 = (r / pm) * s.bn;
+    slice = pair < s.cut.left * s.cut.slices;
   }
   __device__ __forceinline__ bool next(const PairShape& s, PairItem& it) {
-    while (tile < full) {
-      place(s, tile, it);
+    while (tile < s.cut.full) {
+      place_tile(s, tiles_m, tiles_n, tile, it);
       tile += pairs;
+      it.part = -1;
       it.kb0 = 0;
       it.kb1 = num_kb;
       if (s.group_rows != nullptr) {
@@ -85,12 +111,13 @@ struct PairWalk {
       }
       return true;
     }
-    if (lo >= hi) return false;
-    const int t = static_cast<int>(lo / num_kb);
-    place(s, full + t, it);
-    it.kb0 = static_cast<int>(lo - static_cast<long long>(t) * num_kb);
-    it.kb1 = static_cast<int>(min(static_cast<long long>(num_kb), it.kb0 + (hi - lo)));
-    lo += it.kb1 - it.kb0;
+    if (!slice) return false;
+    slice = false;
+    const int t = pair / s.cut.slices, i = pair - t * s.cut.slices;
+    place_tile(s, tiles_m, tiles_n, s.cut.full + t, it);
+    it.part = pair;
+    it.kb0 = num_kb * i / s.cut.slices;
+    it.kb1 = num_kb * (i + 1) / s.cut.slices;
     return true;
   }
 };
@@ -150,8 +177,8 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 template <bool A_MN, bool B_MN, bool OUT_F32>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                 const __grid_constant__ CUtensorMap tmHalf, const __nv_bfloat16* __restrict__ bias, const __grid_constant__ PairShape s,
-                 int add_out, int* status) {
+                 const __grid_constant__ CUtensorMap tmAux /* bf16: boxes of 32 columns; fp32: the workspace of cut tiles */,
+                 const __nv_bfloat16* __restrict__ bias, const __grid_constant__ PairShape s, int add_out, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -348,8 +375,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
-          const CUtensorMap* map = !OUT_F32 && c + 64 > s.bn ? &tmHalf : &tmC;
-          if (add_out)
+          const CUtensorMap* map = !OUT_F32 && c + 64 > s.bn ? &tmAux : &tmC;
+          if (OUT_F32 && it.part >= 0)
+            tma_store_3d(&tmAux, dst, c, row0 - it.m0, it.part);
+          else if (add_out)
             tma_reduce_add_3d(map, dst, col0, row0, it.z);
           else
             tma_store_3d(map, dst, col0, row0, it.z);
@@ -380,6 +409,50 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
 }
 
+// Cut tiles: C (+)= sum of a tile's slices, in K order. Four rows of a tile a block, four slices' loads in flight a thread.
+// Bound by L2: 72 slices of 256 KB are written and read in about 10 us (2560 x 4096 x 9198, 12 tiles in 6 slices: 152 us uncut, 133 cut).
+constexpr int GP_SUM_ROWS = 4;
+template <bool OUT_F32>
+__global__ void __launch_bounds__(256)
+gemm_pair_sum_kernel(const float* __restrict__ parts, void* __restrict__ Cv, const __grid_constant__ PairShape s, int ldc, int add_out) {
+  const int tiles_m = (s.M + 255) / 256, tiles_n = (s.N + s.bn - 1) / s.bn, slices = s.cut.slices;
+  constexpr int BLOCKS = 256 / GP_SUM_ROWS;
+  const int t = blockIdx.x / BLOCKS, r0 = blockIdx.x % BLOCKS * GP_SUM_ROWS;
+  const int vecs = s.bn / 4;
+  const int r = r0 + threadIdx.x / vecs, c = threadIdx.x % vecs * 4;
+  PairItem it;
+  place_tile(s, tiles_m, tiles_n, s.cut.full + t, it);
+  const int row = it.m0 + r, col = it.n0 + c;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (static_cast<int>(threadIdx.x) >= GP_SUM_ROWS * vecs || row >= s.M || col >= s.N) return;
+  const size_t pitch = static_cast<size_t>(256) * s.bn;
+  const float* src = parts + t * slices * pitch + static_cast<size_t>(r) * s.bn + c;
+  float4 acc = *reinterpret_cast<const float4*>(src);
+#pragma unroll 4
+  for (int i = 1; i < slices; ++i) {
+    const float4 v = *reinterpret_cast<const float4*>(src + i * pitch);
+    acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+  }
+  const float out[4] = {acc.x, acc.y, acc.z, acc.w};
+  const size_t at = static_cast<size_t>(row) * ldc + col;
+  if constexpr (OUT_F32) {
+    float* dst = static_cast<float*>(Cv) + at;
+    if (col + 4 <= s.N) {
+      const float4 old = add_out ? *reinterpret_cast<const float4*>(dst) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(dst) = make_float4(old.x + out[0], old.y + out[1], old.z + out[2], old.w + out[3]);
+    } else {
+      for (int i = 0; col + i < s.N; ++i) dst[i] = (add_out ? dst[i] : 0.f) + out[i];
+    }
+  } else {
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(Cv) + at;
+    if (col + 4 <= s.N)
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(out[0], out[1]), pack_bf16x2(out[2], out[3]));
+    else
+      for (int i = 0; col + i < s.N; ++i) dst[i] = __float2bfloat16(out[i]);
+  }
+}
+
 static CUtensorMap pair_out_map(void* C, bool f32, int N, int M, int groups, int ldc, int box_cols) {
   CUtensorMap m;
   const int es = f32 ? 4 : 2;
@@ -394,52 +467,67 @@ static CUtensorMap pair_out_map(void* C, bool f32, int N, int M, int groups, int
   return m;
 }
 
+// OUT_F32: what the kernel writes, in C or in `parts`; c_f32: what C is.
 template <bool A_MN, bool B_MN, bool OUT_F32>
 static cudaError_t launch_pair(const void* A, const void* B, void* C, const void* bias, const PairShape& s, int rows_k, int lda, int ldb, int ldc,
-                               int add, int* status, int num_sms, cudaStream_t stream) {
+                               bool c_f32, int add, float* parts, int* status, cudaStream_t stream) {
+  const PairCut& cut = s.cut;
   CUtensorMap tmA = A_MN ? make_tmap_2d(A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_k, s.M, size_t(lda) * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B)
                          : make_tmap_2d(A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.M, s.K, size_t(lda) * 2, 128, GP_BK, CU_TENSOR_MAP_SWIZZLE_128B);
   CUtensorMap tmB = B_MN ? make_tmap_2d(B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_k, s.N, size_t(ldb) * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B)
                          : make_tmap_2d(B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s.N, s.K, size_t(ldb) * 2, s.bn / 2, GP_BK, CU_TENSOR_MAP_SWIZZLE_128B);
-  CUtensorMap tmC = pair_out_map(C, OUT_F32, s.N, s.M, s.groups, ldc, OUT_F32 ? 32 : 64);
-  CUtensorMap tmHalf = OUT_F32 ? tmC : pair_out_map(C, OUT_F32, s.N, s.M, s.groups, ldc, 32);
+  CUtensorMap tmAux;
+  if (cut.left > 0)
+    tmAux = pair_out_map(parts, true, s.bn, 256, cut.left * cut.slices, s.bn, 32);
+  else
+    tmAux = pair_out_map(C, OUT_F32, s.N, s.M, s.groups, ldc, 32);
+  CUtensorMap tmC = OUT_F32 == c_f32 ? pair_out_map(C, OUT_F32, s.N, s.M, s.groups, ldc, OUT_F32 ? 32 : 64) : tmAux;
   auto kern = gemm_pair_kernel<A_MN, B_MN, OUT_F32>;
   if (cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), GP_SMEM); e != cudaSuccess) {
     set_last_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     return e;
   }
-  const long long tiles = static_cast<long long>((s.M + 255) / 256) * ((s.N + s.bn - 1) / s.bn) * s.groups;
-  long long work = tiles;  // pieces there can be at most
-  if (s.split_last) work = tiles * ((s.K + GP_BK - 1) / GP_BK);
-  const int pairs = static_cast<int>(work < num_sms / 2 ? work : num_sms / 2);
-  cudaError_t le = launch_pdl(kern, dim3(2 * pairs), dim3(GP_THREADS), GP_SMEM, stream, tmA, tmB, tmC, tmHalf,
+  cudaError_t le = launch_pdl(kern, dim3(2 * cut.pairs), dim3(GP_THREADS), GP_SMEM, stream, tmA, tmB, tmC, tmAux,
                               reinterpret_cast<const __nv_bfloat16*>(bias), s, add, status);
+  if (le == cudaSuccess && cut.left > 0)
+    le = launch_pdl(c_f32 ? gemm_pair_sum_kernel<true> : gemm_pair_sum_kernel<false>, dim3(cut.left * (256 / GP_SUM_ROWS)), dim3(256), 0, stream,
+                    static_cast<const float*>(parts), C, s, ldc, add);
   if (le != cudaSuccess) set_last_error(std::string("gemm_pair launch: ") + cudaGetErrorString(le));
   return le;
 }
 
 }  // namespace sb
 
-// Operands as sb_gemm_bf16. `bn`: tile width, a multiple of 32 from 128 to 256. `add` = 1: C (fp32) is added to. `split_last` = 1: the last
-// wave of tiles is cut along K (add only). `groups` > 1 (a_mn and b_mn only, fp32 C): C is [groups, M, N] and group e sums over the rows
+// Operands as sb_gemm_bf16. `bn`: tile width, a multiple of 32 from 128 to 256. `add` = 1: C (fp32) is added to. `split_last` = 1: the tiles
+// behind the last full wave of num_sms / 2 are cut along K where there are pairs and k-blocks for it; `parts` is then scratch of num_sms / 2 *
+// 256 * bn floats, 16-byte aligned. (A bf16 C: only with fewer tiles than a wave, and at least 16 k-blocks.) `groups` > 1 (a_mn and b_mn
+// only, fp32 C): C is [groups, M, N] and group e sums over the rows
 // group_start[e] .. + group_rows[e] of A and B, which hold K rows in all; group_start are multiples of 64 and the rows behind a group's
-// last, up to a multiple of 64, are zero. C's base and pitch are multiples of 16 bytes.
+// last, up to a multiple of 64, are zero. C's base and pitch are multiples of 16 bytes (8 where a bf16 C is cut).
 extern "C" int sb_gemm_pair(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
-                            int b_mn, int out_f32, int add, int bn, int split_last, int groups, const int* group_start,
+                            int b_mn, int out_f32, int add, int bn, int split_last, float* parts, int groups, const int* group_start,
                             const int* group_rows, int* status, int num_sms, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || groups <= 0) return 0;
   const bool grouped = group_start != nullptr;
-  if (bn < 128 || bn > 256 || bn % 32 || (a_mn && !b_mn) || (add && !out_f32) || (split_last && (!add || grouped)) ||
-      (groups > 1 && !grouped) || (grouped && (!a_mn || !b_mn || !out_f32 || group_rows == nullptr || bias != nullptr)) || num_sms < 2 ||
-      (reinterpret_cast<uintptr_t>(C) & 15) || (size_t(ldc) * (out_f32 ? 4 : 2)) % 16) {
-    sb::set_last_error("sb_gemm_pair: shape, layout or alignment not supported");
+  if (bn < 128 || bn > 256 || bn % 32 || (a_mn && !b_mn) || (add && !out_f32) || (split_last && grouped) || (groups > 1 && !grouped) ||
+      (grouped && (!a_mn || !b_mn || !out_f32 || group_rows == nullptr || bias != nullptr)) || num_sms < 2) {
+    sb::set_last_error("sb_gemm_pair: shape or layout not supported");
     return (int)cudaErrorInvalidValue;
   }
-  const sb::PairShape s{M, N, K, bn, groups, group_start, group_rows, split_last};
+  const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + bn - 1) / bn) * groups;
+  const sb::PairCut cut = sb::cut_last_wave(tiles, (K + sb::GP_BK - 1) / sb::GP_BK, num_sms, split_last != 0);
+  const int align = cut.left > 0 && !out_f32 ? 8 : 16;
+  if (reinterpret_cast<uintptr_t>(C) % align || (size_t(ldc) * (out_f32 ? 4 : 2)) % align ||
+      (cut.left > 0 && (parts == nullptr || (reinterpret_cast<uintptr_t>(parts) & 15) || (!out_f32 && cut.full > 0)))) {
+    sb::set_last_error("sb_gemm_pair: alignment, or a cut without its workspace, or of a bf16 output of more than a wave");
+    return (int)cudaErrorInvalidValue;
+  }
+  const sb::PairShape s{M, N, K, bn, groups, group_start, group_rows, cut};
+  const bool f32 = out_f32 || cut.left > 0;
   try {
 #define SB_CASE(AM, BM_, OF)                   \
-  if ((a_mn != 0) == AM && (b_mn != 0) == BM_ && (out_f32 != 0) == OF) \
-    return (int)sb::launch_pair<AM, BM_, OF>(A, B, C, bias, s, K, lda, ldb, ldc, add, status, num_sms, stream);
+  if ((a_mn != 0) == AM && (b_mn != 0) == BM_ && f32 == OF) \
+    return (int)sb::launch_pair<AM, BM_, OF>(A, B, C, bias, s, K, lda, ldb, ldc, out_f32 != 0, add, parts, status, stream);
     SB_CASE(false, false, false)
     SB_CASE(false, false, true)
     SB_CASE(false, true, false)

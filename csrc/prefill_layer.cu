@@ -8,7 +8,7 @@
 extern "C" {
 int sb_rmsnorm_fwd(const void*, const void*, const void*, void*, void*, float*, int, int, float, cudaStream_t);
 int sb_rmsnorm_fwd_f32x(const float*, const void*, const void*, void*, void*, float*, int, int, float, cudaStream_t);
-int sb_gemm_pair(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, int, int, const int*,
+int sb_gemm_pair(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, int, float*, int, const int*,
                  const int*, int*, int, cudaStream_t);
 int sb_gemm_bf16_splitk(const void*, const void*, void*, const void*, int, int, int, int, int, int, int, int, int, int, int, int, int*, int,
                         cudaStream_t);
@@ -42,7 +42,7 @@ static int project(const PrefillLayer& p, int which, const void* a, const void* 
                    cudaStream_t s) {
   const int* plan = p.plan[which];
   if (plan[0] > 0)
-    return sb_gemm_pair(a, w, out, bias, p.T, N, K, K, K, N, 0, 0, f32, 0, plan[0], 0, 1, nullptr, nullptr, p.status, p.num_sms, s);
+    return sb_gemm_pair(a, w, out, bias, p.T, N, K, K, K, N, 0, 0, f32, 0, plan[0], 0, nullptr, 1, nullptr, nullptr, p.status, p.num_sms, s);
   if (plan[2] > 1)  // the slices are added up in the output
     if (cudaError_t e = cudaMemsetAsync(out, 0, static_cast<size_t>(p.T) * N * 4, s); e != cudaSuccess) return (int)e;
   return sb_gemm_bf16_splitk(a, w, out, bias, p.T, N, K, K, K, N, 0, 0, f32, 0, plan[1], plan[2], p.status, p.num_sms, s);

@@ -95,40 +95,58 @@ def _pick_splitk(M: int, N: int, K: int, bn: int, sms: int = 148) -> int:
     return max(1, min(kb // 8, sms // tiles))
 
 
+_PAIR_RATES = ((256, 1.0), (224, 0.92), (192, 0.85), (128, 0.65))  # tile width, rate per column
+
+
+def _cut_slices(rest: int, kb: int, pairs: int) -> int:
+    """Slices of K of each of the ``rest`` tiles behind the last full wave (``cut_last_wave`` in ``csrc/gemm_pair_sm100.cu``); 1: uncut."""
+    return max(1, min(pairs // rest, kb // 8)) if rest else 1
+
+
 @functools.lru_cache(maxsize=4096)
-def _pick_pair(M: int, N: int, K: int, split_last: bool, sms: int = 148) -> int:
-    """Tile width of the kernel that works on pairs of SMs (``csrc/gemm_pair_sm100.cu``), 0 where the one-SM kernel is better.
+def _pick_pair(M: int, N: int, K: int, accumulate: bool, sms: int = 148) -> tuple[int, bool]:
+    """Tile width of the kernel that works on pairs of SMs (``csrc/gemm_pair_sm100.cu``) and whether to cut its last wave; width 0 where the
+    one-SM kernel is better.
 
     A wave model again, in widths of a 256-wide tile at full rate. Measured (9198 x 19456 x 2560 and the like): pairs run a 256-wide
     tile 1.12 times as fast as one SM; narrower tiles reach 0.92 (224 wide), 0.85 (192) and 0.65 (128) of its rate per column, and pay
     where they fit N (896 = 4 x 224) or fill a wave. A pair's launch is about 2 us longer (two CTAs meet before and after), the
-    time of 1900 columns of one k-block: 397 x 9728 x 896 takes 22.7 us on single SMs, 23.6 on pairs; 15800 x 9728 x 896 217 and 193."""
+    time of 1900 columns of one k-block: 397 x 9728 x 896 takes 22.7 us on single SMs, 23.6 on pairs; 15800 x 9728 x 896 217 and 193.
+
+    Outputs that are added to (weight gradients: both operands are read across K, and a narrower tile takes as long as a wide one: 9728 x
+    896 x 9198 152 us with 256 wide tiles, 153 with 224, 155 with 192): up to 8 k-blocks their traffic bounds the call, and single SMs move it faster (397 rows, 6144 x 2560: 26.7 us
+    and 28.3 on pairs; 19456 x 2560: 92 and 95; 700 rows: 33.2 and 30.9, 101 and 101); with less than a wave of tiles the uniform slices of
+    the one-SM kernel are faster (896 x 896 x 15800: 32 and 40). A cut takes 4 us and 0.13 us a slice, for the workspace and its second launch:
+    9728 x 896 x 15800 258 us uncut, 211 cut; 2560 x 4096 x 9198 152 and 133; 4096 x 4096 x 2048 59.8 and 66.4."""
     if M == 0 or N == 0 or K == 0:
-        return 0
+        return 0, False
     kb = -(-K // 64)
     pairs = sms // 2
-    best, width = 1e30, 0
-    for bn, rate in ((256, 1.0), (224, 0.92), (192, 0.85), (128, 0.65)):
+    best, width, cut = 1e30, 0, False
+    if accumulate and kb < 9:
+        return 0, False
+    for bn, rate in _PAIR_RATES:
+        if accumulate and bn < 256:
+            break
         tiles = -(-M // 256) * -(-N // bn)
-        if tiles < pairs // 2 and not split_last:  # one tile's chain of k-blocks bounds the call: smaller tiles on single SMs, or slices of K
+        if tiles < (pairs if accumulate else pairs // 2):  # one tile's chain of k-blocks bounds the call: smaller tiles on single SMs, or slices of K
             continue
-        if split_last and tiles >= pairs:  # with fewer tiles the uniform slices of the one-SM kernel are faster (35 and 39 us: 896 x 896 x 15800)
-            waves = tiles / pairs
-        elif split_last:
-            continue
-        else:
-            waves = -(-tiles // pairs)
-        cost = waves * bn / rate + 1900.0 / kb
-        if cost < best:
-            best, width = cost, bn
+        forms = [(-(-tiles // pairs), 0.0, False)]
+        slices = _cut_slices(tiles % pairs, kb, pairs)
+        if accumulate and slices > 1:
+            forms.append((tiles // pairs + 1 / slices, 2640.0 + 86.0 * (tiles % pairs) * slices, True))
+        for waves, fixed, cuts in forms:
+            cost = waves * bn / rate + (fixed + (600.0 if accumulate else 1900.0)) / kb
+            if cost < best:
+                best, width, cut = cost, bn, cuts
     t128 = -(-M // 128)
     single = min(-(-(t128 * -(-N // 256)) // sms) * 256 / 0.88, -(-(t128 * -(-N // 128)) // sms) * 128 / 0.62)
-    return width if best < single else 0
+    return (width, cut) if best < single else (0, False)
 
 
 def gemm_plan(M: int, N: int, K: int, f32: bool, sms: int) -> tuple[int, int, int]:
     """What ``gemm`` does with row-major operands and a new output: (width on pairs of SMs or 0, width on one SM, slices of K)."""
-    width, bn = _pick_pair(M, N, K, False, sms), _pick_bn(M, N)
+    (width, _), bn = _pick_pair(M, N, K, False, sms), _pick_bn(M, N)
     return width, bn, _pick_splitk(M, N, K, bn, sms) if f32 and N % 4 == 0 else 1
 
 
@@ -167,18 +185,22 @@ def gemm(a, b, *, a_mn=False, b_mn=False, bias=None, out=None, out_dtype=None, a
     if b.stride(-1) != 1:
         b = b.contiguous()
     if bn is None and splitk is None and (b_mn or not a_mn):
-        sms, split_last = _lib.sm_count(a.device), accumulate and not BATCH_INVARIANT
-        width = _pick_pair(M, N, K, split_last, sms)
-        res = _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms) if width else None
+        sms = _lib.sm_count(a.device)
+        width, cut = _pick_pair(M, N, K, accumulate, sms)
+        res = _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, cut and not BATCH_INVARIANT, M, N, K, sms) if width else None
         if res is not None:
             return res
-    if out_dtype == torch.bfloat16 and bn is None and splitk is None and K >= 16384 and N % 4 == 0 and not accumulate:
-        # a bf16 output of few tiles over a very long K (gradients of few rows behind a head): sums of K slices in fp32, then rounded.
-        # 265 x 896 x 151936: 661 -> 120 us, 100 x 2560 x 16384: 80 -> 34. The fill and the conversion cost about 5.
-        slices = _pick_splitk(M, N, K, 128, _lib.sm_count(a.device))
-        if slices > 1:
-            res = gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, out_dtype=torch.float32, bn=128, splitk=slices)
-            return res.to(out_dtype) if out is None else out.copy_(res)
+    if out_dtype == torch.bfloat16 and bn is None and splitk is None and K >= 16384 and (b_mn or not a_mn) and not BATCH_INVARIANT:
+        # A bf16 output of few tiles over a very long K (gradients of few rows behind a head): K slices, summed in order, then rounded. 265 x
+        # 896 x 151936: 670 us in one chain, 132 cut; 100 x 2560 x 16384: 80 and 29. Shorter sums would gain too (397 x 896 x 9728: 47 and
+        # 18); they keep the one chain of the batch-invariant mode, and with it the bits that a layer has there.
+        sms = _lib.sm_count(a.device)
+        width = min((-(-N // w) * w / rate, w) for w, rate in _PAIR_RATES)[1]
+        tiles = -(-M // 256) * -(-N // width)
+        if tiles < sms // 2 and _cut_slices(tiles, -(-K // 64), sms // 2) > 1:
+            res = _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, False, width, True, M, N, K, sms)
+            if res is not None:
+                return res
     bn = bn or _pick_bn(M, N)
     can_split = out_dtype == torch.float32 and (accumulate or (out is None and N % 4 == 0))  # TMA reduce-add: 16-byte rows
     if splitk is None:
@@ -215,7 +237,8 @@ def _empty_product(bias, out, out_dtype, accumulate, M, N, device):
 
 
 def _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_last, M, N, K, sms):
-    """None: an output that TMA cannot write (base or pitch not a multiple of 16 bytes)."""
+    """``split_last``: cut the tiles behind the last full wave along K (a bf16 output: only where there are less than a wave). None: an output
+    that the kernel cannot write (base or pitch not a multiple of 16 bytes, of 8 for a cut bf16 output)."""
     if out is None:
         assert not accumulate
         out = torch.empty(M, N, dtype=out_dtype, device=a.device)
@@ -223,11 +246,13 @@ def _gemm_pair(a, b, a_mn, b_mn, bias, out, out_dtype, accumulate, width, split_
     assert not (accumulate and out.dtype != torch.float32), "accumulate needs an fp32 output"
     lda, ldb, ldc = a.stride(0), b.stride(0), out.stride(0)
     assert lda % 8 == 0 and ldb % 8 == 0, "TMA needs 16-byte row pitches (multiples of 8 bf16)"
-    if out.data_ptr() % 16 or (ldc * out.element_size()) % 16:
-        return None
     f32 = out.dtype == torch.float32
+    align = 8 if split_last and not f32 else 16
+    if out.data_ptr() % align or (ldc * out.element_size()) % align:
+        return None
+    parts = torch.empty(sms // 2, 256, width, dtype=torch.float32, device=a.device) if split_last else None  # of cut tiles: one slice a pair
     rc = _lib.lib().sb_gemm_pair(
-        P(a), P(b), P(out), P(bias), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32), int(accumulate), width, int(split_last), 1,
+        P(a), P(b), P(out), P(bias), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), int(f32), int(accumulate), width, int(split_last), P(parts), 1,
         None, None, P(_lib.status_word(a.device)), sms, _lib.stream(),
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_pair")

@@ -72,7 +72,7 @@ _SIGS = {
     "sb_gemm_fp8_grouped": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P, I, P],
     "sb_gemm_bf16_grouped": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, I, P],
     "sb_gemm_bf16_splitk": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, I, P],
-    "sb_gemm_pair": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P, P, I, P],
+    "sb_gemm_pair": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, P, I, P, P, P, I, P],
     "sb_flash_fwd": [P] * 6 + [I] * 12 + [F, P, P],
     "sb_flash_bwd": [P] * 11 + [I, P] + [I] * 17 + [F, P, P],
     "sb_prefill_layer": [P, P],

@@ -442,7 +442,7 @@ def _add_weight_grads(dy: torch.Tensor, x: torch.Tensor, lay, grads: list[torch.
         return False
     width = min((256, 224, 192, 128), key=lambda bn: -(-N // bn) * bn / {256: 1.0, 224: 0.92, 192: 0.85, 128: 0.65}[bn])  # rates: ops._pick_pair
     rc = _lib.lib().sb_gemm_pair(
-        P(dy), P(x), P(out), None, M, N, lay.rows_padded, dy.stride(0), x.stride(0), N, 1, 1, 1, 1, width, 0, E, P(lay.expert_rows[0]),
+        P(dy), P(x), P(out), None, M, N, lay.rows_padded, dy.stride(0), x.stride(0), N, 1, 1, 1, 1, width, 0, None, E, P(lay.expert_rows[0]),
         P(lay.expert_rows[1]), P(_lib.status_word(dy.device)), _lib.sm_count(dy.device), _lib.stream(),
     )  # fmt: skip
     _lib.check(rc, "sb_gemm_pair")

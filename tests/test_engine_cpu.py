@@ -389,5 +389,5 @@ def test_plans_of_empty_products():
     from slime_b200 import ops
 
     for M, N, K in ((9728, 896, 0), (151936, 896, 0), (2560, 4096, 0), (0, 896, 151936), (0, 896, 896), (128, 0, 4096), (0, 0, 0)):
-        assert all(ops._pick_pair(M, N, K, cut) == 0 for cut in (False, True))
+        assert all(ops._pick_pair(M, N, K, add) == (0, False) for add in (False, True))
         assert all(ops._pick_splitk(M, N, K, bn) == 1 for bn in (128, 256)) and ops.gemm_plan(M, N, K, True, 148)[2] == 1

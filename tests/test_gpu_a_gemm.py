@@ -123,3 +123,32 @@ def test_products_over_nothing(kernels, out, inp):
     assert ops.gemm(a, c, b_mn=True).shape == (0, 896)  # the gradient of no rows behind a head
     empty, bias = torch.empty(5, 0, device="cuda", dtype=torch.bfloat16), torch.randn(7, device="cuda").bfloat16()
     assert torch.equal(ops.gemm(empty, empty.new_empty(7, 0), bias=bias), bias.expand(5, 7))
+
+
+@pytest.mark.parametrize("M,N,K", [(9728, 896, 15800), (2560, 4096, 9198), (264, 24904, 1096), (9472, 512, 72)])
+def test_weight_gradients_are_the_same_on_every_run(kernels, M, N, K):
+    """Outputs of more than a wave of tiles, added to: the ranges of a cut tile are summed in one order. Against 64 bits: each of K / 16 steps
+    of a sum of at most 4 sqrt(K) may lose an ulp, 2^-23 of it."""
+    torch.manual_seed(K)
+    dy, x = (torch.randn(K, n, device="cuda").bfloat16() for n in (M, N))
+    start = torch.randn(M, N, device="cuda")
+    runs = [ops.gemm(dy, x, a_mn=True, b_mn=True, out=start.clone(), accumulate=True) for _ in range(8)]
+    assert all(torch.equal(runs[0], r) for r in runs[1:])
+    for cut in (False, True):  # whatever the plan is
+        runs = [ops._gemm_pair(dy, x, True, True, None, start.clone(), None, True, 256, cut, M, N, K, 148) for _ in range(8)]
+        assert all(torch.equal(runs[0], r) for r in runs[1:])
+        torch.testing.assert_close((runs[0] - start).double(), dy.double().t() @ x.double(), rtol=1e-5, atol=K / 16 * 2.0**-23 * 4 * K**0.5 + 2e-6)
+
+
+@pytest.mark.parametrize("M,N,K", [(265, 896, 151936), (1, 8, 16384), (130, 900, 20000), (257, 4, 16390)])
+def test_few_rows_over_a_long_sum_are_the_same_on_every_run(kernels, M, N, K):
+    """A bf16 output whose sums are cut along K, written through any row view: one order, one rounding."""
+    torch.manual_seed(M)
+    a, b = torch.randn(M, -(-K // 8) * 8, device="cuda").bfloat16()[:, :K], (torch.randn(K, N + (-N) % 8, device="cuda") * 0.02).bfloat16()[:, :N]
+    bias = torch.randn(N, device="cuda").bfloat16()
+    wide = torch.zeros(M, N + 4, device="cuda", dtype=torch.bfloat16)
+    runs = [ops.gemm(a, b, b_mn=True, bias=bias) for _ in range(8)]
+    assert all(torch.equal(runs[0], r) for r in runs[1:])
+    ops.gemm(a, b, b_mn=True, bias=bias, out=wide[:, :N])
+    assert torch.equal(wide[:, :N], runs[0]) and (wide[:, N:] == 0).all()
+    torch.testing.assert_close(runs[0].double(), a.double() @ b.double() + bias.double(), rtol=2**-8, atol=1e-3)
