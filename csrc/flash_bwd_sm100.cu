@@ -452,7 +452,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
   if (warp == 1) tmem_dealloc(tmem_base, S::TMEM_COLS);
 }
 
-// dV, dK = sum over the parts, in part order, of the rows inside a segment: CTA (tile, 0: dV, 1: dK), one 8-column vector per thread and step.
+// dV, dK = sum over the parts, in part order, of the rows inside a segment: CTA (tile, 0: dV, 1: dK, eight rows of the tile), one 8-column
+// vector per thread and step. Parts are taken where there are few tiles, so a tile has many CTAs here (one took 50 us for 128 rows of 1024
+// columns in four parts).
+constexpr int FB_SUM_ROWS = 8;
 __global__ void __launch_bounds__(256)
 flash_bwd_sum_kernel(const float* __restrict__ part_out, __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ dk, const int* __restrict__ seg,
                      int nseg, int parts, int Tk, int width, int dv_stride, int dk_stride) {
@@ -469,13 +472,14 @@ flash_bwd_sum_kernel(const float* __restrict__ part_out, __nv_bfloat16* __restri
   }
   __syncthreads();
   if (work[0] < 0) return;
-  const int t0 = work[1] * FB_T, rows = min(FB_T, seg[4 * work[0] + 3] - t0), row0 = seg[4 * work[0] + 2] + t0;
+  const int t0 = work[1] * FB_T + blockIdx.z * FB_SUM_ROWS, rows = min(FB_SUM_ROWS, seg[4 * work[0] + 3] - t0), row0 = seg[4 * work[0] + 2] + t0;
   const int a = blockIdx.y, vecs = width / 8;
   __nv_bfloat16* dst = a == 0 ? dv : dk;
   const int stride = a == 0 ? dv_stride : dk_stride;
   for (int i = threadIdx.x; i < rows * vecs; i += 256) {
     const int r = row0 + i / vecs, c = (i % vecs) * 8;
     float s[8] = {};
+#pragma unroll 4
     for (int p = 0; p < parts; ++p) {
       const float4* src = reinterpret_cast<const float4*>(part_out + ((static_cast<size_t>(p) * 2 + a) * Tk + r) * width + c);
       const float4 x = src[0], y = src[1];
@@ -514,7 +518,7 @@ static int launch_flash_bwd(const void* q, const void* k, const void* v, const v
                                Hkv, Tk, parts, max_k_tiles, dv_stride, dk_stride, stat_stride, scale, status);
     if (e != cudaSuccess) return (int)e;
     if (parts > 1) {
-      e = launch_pdl(flash_bwd_sum_kernel, dim3(max_k_tiles, 2), dim3(256), 0, s, (const float*)part_out, (bf16*)dv, (bf16*)dk, seg, nseg, parts,
+      e = launch_pdl(flash_bwd_sum_kernel, dim3(max_k_tiles, 2, FB_T / FB_SUM_ROWS), dim3(256), 0, s, (const float*)part_out, (bf16*)dv, (bf16*)dk, seg, nseg, parts,
                      Tk, Hkv * D, dv_stride, dk_stride);
       if (e != cudaSuccess) return (int)e;
     }

@@ -97,10 +97,30 @@ def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, 
     return out, lse
 
 
-def _key_parts(ctas: int, group: int, sms: int) -> int:
-    """CTAs that share the query heads of one (key tile, kv head) in the backward: enough to give every SM about three, so that the
-    long tiles of one SM find company on the others; the parts are summed in fp32 afterwards."""
-    return max(1, min(group, -(-3 * sms // max(ctas, 1))))
+def _key_parts(Tq: int, Tk: int, nseg: int, Hq: int, Hkv: int, D: int, sms: int) -> int:
+    """CTAs that share the query heads of one (key tile, kv head) in the backward.
+
+    A CTA of the dK / dV pass takes about 0.8 us (head width 64; 1.0 us: 128) for each query block of each of its heads, and one such step to
+    begin and end. The pass takes as long as its longest CTA, that of the first keys, or as all of them on all SMs. Parts shorten the longest one, but
+    their fp32 sums are written, read and added up by a launch of their own: 4 us and 16 bytes an element of dK at 6 TB/s. The lengths
+    are on the device; equal ones are assumed here. Best of all parts and this rule, us, all launches of the backward: 397 rows, 14 / 2
+    heads of 64, seven parts 29 (one part: 67); 16 x 128 rows, 32 / 8 heads of 128, one part 55 (two parts 78); 2048 rows two parts 190 (254)."""
+    if not (Tq and Tk and nseg):
+        return 1
+    group, heads = Hq // Hkv, Hq
+    rows, keys = -(-Tq // nseg), -(-Tk // nseg)
+    blocks, tiles = -(-rows // 64), -(-keys // 128)  # of one segment
+    hidden = max(0, tiles - 1 - (keys - rows) // 128)  # tiles behind the first query's last key: the n-th of them is not seen by 2 n blocks
+    steps = max(blocks * tiles - hidden * (hidden + 1), tiles) * nseg * heads
+    step_us = 0.8 if D == 64 else 1.0
+    best, parts = math.inf, 1
+    for p in range(1, group + 1):
+        t = step_us * max(-(-group // p) * blocks + 1, (steps + nseg * tiles * Hkv * p) / sms)
+        if p > 1:
+            t += 4.0 + p * Tk * Hkv * D * 16 / 6e6
+        if t < best:
+            best, parts = t, p
+    return parts
 
 
 def flash_bwd(q, k, v, o, d_o, lse, seg, scale, dq=None, dk=None, dv=None):
@@ -117,7 +137,7 @@ def flash_bwd(q, k, v, o, d_o, lse, seg, scale, dq=None, dk=None, dv=None):
     delta = torch.empty_like(lse)
     nseg = seg.shape[0]
     k_tiles = -(-Tk // 128) + nseg
-    parts = _key_parts(k_tiles * Hkv, Hq // Hkv, _lib.sm_count(q.device))
+    parts = _key_parts(Tq, Tk, nseg, Hq, Hkv, D, _lib.sm_count(q.device))
     partial = torch.empty(parts, 2, Tk, Hkv * D, dtype=torch.float32, device=q.device) if parts > 1 else None
     rc = _lib.lib().sb_flash_bwd(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), lse.data_ptr(), delta.data_ptr(),

@@ -391,3 +391,13 @@ def test_plans_of_empty_products():
     for M, N, K in ((9728, 896, 0), (151936, 896, 0), (2560, 4096, 0), (0, 896, 151936), (0, 896, 896), (128, 0, 4096), (0, 0, 0)):
         assert all(ops._pick_pair(M, N, K, add) == (0, False) for add in (False, True))
         assert all(ops._pick_splitk(M, N, K, bn) == 1 for bn in (128, 256)) and ops.gemm_plan(M, N, K, True, 148)[2] == 1
+
+
+def test_parts_of_the_attention_backward():
+    """One part where there is nothing to share or CTAs enough, several for one long sequence of few heads, never more than the group has heads."""
+    from slime_b200.ops.attention import _key_parts
+
+    assert _key_parts(0, 0, 0, 14, 2, 64, 148) == _key_parts(5, 0, 2, 14, 2, 64, 148) == 1
+    assert _key_parts(16, 16, 1, 32, 8, 128, 148) == _key_parts(2048, 2048, 16, 32, 8, 128, 148) == _key_parts(15800, 15800, 19, 14, 2, 64, 148) == 1
+    assert _key_parts(4096, 4096, 1, 14, 2, 64, 148) > 1 and _key_parts(397, 397, 1, 14, 2, 64, 148) == 7
+    assert all(1 <= _key_parts(t, c, n, 8 * g, 8, 128, 148) <= g for t in (1, 300, 9000) for c in (t, t + 5000) for n in (1, 7) for g in (1, 3, 8))

@@ -188,3 +188,28 @@ def test_flash_forward_pairs_of_tiles(kernels, pairs, D):
         s = torch.einsum("thd,shd->hts", q[qo : qo + ql].double(), k[ko : ko + kl].double().repeat_interleave(Hq // Hkv, 1)) * D**-0.5
         s = s.masked_fill(~torch.ones(ql, kl, dtype=torch.bool, device="cuda").tril(kl - ql), -math.inf)
         assert float((lse[:, qo : qo + ql] - s.logsumexp(-1)).abs().max()) < 1e-4 * max(1.0, float(s.amax()))
+
+
+@pytest.mark.parametrize("parts", [2, 3, 4, 7])
+@pytest.mark.parametrize("lens,Hkv,D", [([1 + 37 * i % 191 for i in range(70)], 2, 64), ([7, 63, 64, 65, 127, 129, 193], 1, 128), ([300], 8, 128)])
+def test_flash_backward_in_any_number_of_parts(kernels, monkeypatch, parts, lens, Hkv, D):
+    """dK and dV as sums of fp32 parts against one part: sums in another order, one rounding to bf16 (2^-8); dQ has no parts. Rows outside
+    every segment stay as they are."""
+    from slime_b200.ops import _lib, attention
+
+    torch.manual_seed(parts)
+    T, Hq = sum(lens) + 3, 7 * Hkv
+    q, d_o = (torch.randn(T, Hq, D, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(T, Hkv, D, device="cuda").bfloat16() for _ in range(2))
+    seg = attention.segments_from_cu_seqlens(torch.tensor([0] + lens, device="cuda").cumsum(0))
+    out, lse = attention.flash_fwd(q, k, v, seg, D**-0.5, zero_uncovered=True)
+    got = []
+    for p in (1, parts):
+        monkeypatch.setattr(attention, "_key_parts", lambda *a: p)
+        grads = [torch.full_like(t, 5.0) for t in (q, k, v)]
+        got.append(attention.flash_bwd(q, k, v, out, d_o, lse, seg, D**-0.5, *grads))
+    _lib.check_status("cuda")
+    assert torch.equal(got[0][0], got[1][0])
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert (b[-3:] == 5).all()
+        torch.testing.assert_close(a, b, rtol=2**-7, atol=2.0**-16 * float(a[:-3].abs().max()))
