@@ -11,7 +11,8 @@
 //
 // One CTA = 256 query rows of one head, as two tiles of 128. 10 warps: warp 0 issues TMA loads (Q once, K / V tiles of 128 keys
 // through a 2-stage ring that both tiles read), warp 1 owns TMEM and issues tcgen05.mma, and each query tile g has a softmax group of
-// four warps: thread r owns query row r (= TMEM lane r).
+// four warps: thread r owns query row r (= TMEM lane r). Where the machine is not filled by that, one CTA = 128 rows: one tile and one
+// softmax group, the scores of the next key tile computed beside the softmax of this one (see launch_flash_fwd_tiles).
 //
 //   S_g  = Q_g K_j^T          M 128, N 128, K D        TMEM
 //   P_g  = 2^(S_g*c - m)      TMEM -> registers -> bf16 over the scores it came from (the A operand of the next product)
@@ -32,19 +33,20 @@
 
 namespace sb {
 
-constexpr int FA_BM = 128;       // query rows of one tile; a CTA has two
+constexpr int FA_BM = 128;       // query rows of one tile; a CTA has one or two
 constexpr int FA_BN = 128;       // keys per tile
-constexpr int FA_THREADS = 320;  // TMA warp, MMA warp, 2 x 4 softmax warps
 constexpr int FA_KV_STAGES = 2;
 
-template <int D>
+template <int D, int TILES>
 struct FaSmem {
+  static constexpr int THREADS = 64 + 128 * TILES;    // TMA warp, MMA warp, four softmax warps a tile
   static constexpr int NCH = D / 64;                  // 128-byte chunks of the head dim
   static constexpr int Q_BYTES = FA_BM * 128 * NCH;   // one query tile, [NCH][128 rows][128 B]; its output is staged here at the end
   static constexpr int KV_BYTES = FA_BN * 128 * NCH;  // one K or V tile
   static constexpr int BAR_BYTES = 256;
-  static constexpr int TOTAL = 2 * Q_BYTES + 2 * FA_KV_STAGES * KV_BYTES + BAR_BYTES + 1024;  // +1024: alignment
-  static constexpr int TMEM_COLS = 512;  // S_0 @0, S_1 @128 (P_g over the first 64 columns of S_g), O_0 @256, O_1 @256 + D
+  static constexpr int TOTAL = TILES * Q_BYTES + 2 * FA_KV_STAGES * KV_BYTES + BAR_BYTES + 1024;  // +1024: alignment
+  // S_0 @0, S_1 @128 (P over the first 64 columns of its S), O_0 @256, O_1 @256 + D. One tile: S_b holds the scores of key tiles j % 2 = b.
+  static constexpr int TMEM_COLS = 512;
 };
 
 __device__ __forceinline__ float fa_exp2(float x) {
@@ -57,30 +59,30 @@ __device__ __forceinline__ void fa_named_barrier(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-template <int D>
-__global__ void __launch_bounds__(FA_THREADS, 1)
+template <int D, int TILES>
+__global__ void __launch_bounds__(FaSmem<D, TILES>::THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
                  const int* __restrict__ seg, int nseg, int Hq, int Hkv, int tiles, int out_stride, int lse_stride, float scale,
                  int* status) {
-  using S = FaSmem<D>;
+  using S = FaSmem<D, TILES>;
   constexpr int NCH = S::NCH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;                                  // [2 tiles]
-  uint8_t* sK = sQ + 2 * S::Q_BYTES;
+  uint8_t* sQ = smem;                                  // [TILES]
+  uint8_t* sK = sQ + TILES * S::Q_BYTES;
   uint8_t* sV = sK + FA_KV_STAGES * S::KV_BYTES;
   uint64_t* q_full = reinterpret_cast<uint64_t*>(sV + FA_KV_STAGES * S::KV_BYTES);
   uint64_t* k_full = q_full + 1;
   uint64_t* k_empty = k_full + FA_KV_STAGES;
   uint64_t* v_full = k_empty + FA_KV_STAGES;
   uint64_t* v_empty = v_full + FA_KV_STAGES;
-  uint64_t* s_full = v_empty + FA_KV_STAGES;  // [2 groups] scores of a tile are in TMEM, and every earlier product has finished
-  uint64_t* p_full = s_full + 2;              // [2 groups] P is in TMEM (4 arrivals)
-  uint64_t* o_full = p_full + 2;              // [2 groups] the group's last product has finished
+  uint64_t* s_full = v_empty + FA_KV_STAGES;  // [2 score buffers] scores are in TMEM, and every product issued before them has finished
+  uint64_t* p_full = s_full + 2;              // [groups] P is in TMEM (4 arrivals)
+  uint64_t* o_full = p_full + 2;              // [groups] the group's last product has finished (one tile: each product)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* work = reinterpret_cast<int*>(tmem_slot + 2);  // [0] segment or -1, [1] pair of tiles in the segment
+  int* work = reinterpret_cast<int*>(tmem_slot + 2);  // [0] segment or -1, [1] number of the TILES tiles in the segment
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int h = blockIdx.x % Hq;
@@ -113,7 +115,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   pdl_launch_dependents();
   if (warp == 0) {
     int pair;
-    const int found = segment_of_tile(seg, nseg, 1, 2 * FA_BM, tiles - 1 - static_cast<int>(blockIdx.x / Hq), pair);
+    const int found = segment_of_tile(seg, nseg, 1, TILES * FA_BM, tiles - 1 - static_cast<int>(blockIdx.x / Hq), pair);
     if (lane == 0) {
       work[0] = found;
       work[1] = pair;
@@ -126,22 +128,22 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int sidx = work[0];
   if (sidx >= 0) {
     const int q_off = seg[4 * sidx], q_len = seg[4 * sidx + 1], k_off = seg[4 * sidx + 2], k_len = seg[4 * sidx + 3];
-    const int q0 = work[1] * 2 * FA_BM;          // first query row of this CTA inside the segment
+    const int q0 = work[1] * TILES * FA_BM;      // first query row of this CTA inside the segment
     const int shift = k_len - q_len;             // query i sees keys j <= shift + i
-    // key tiles of the two query tiles (none for a second tile that lies past the segment)
+    // key tiles of the query tiles (none for a second tile that lies past the segment)
     auto key_tiles = [&](int g) {
       const int r0 = q0 + g * FA_BM;
       return r0 < q_len ? (max(min(k_len, shift + r0 + FA_BM), 0) + FA_BN - 1) / FA_BN : 0;
     };
-    const int n_of[2] = {key_tiles(0), key_tiles(1)};
+    const int n_of[2] = {key_tiles(0), TILES == 2 ? key_tiles(1) : 0};
     const int n_kv = max(n_of[0], n_of[1]);
 
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       if (lane == 0 && n_kv > 0) {
-        mbar_arrive_expect_tx(q_full, 2 * S::Q_BYTES);
+        mbar_arrive_expect_tx(q_full, TILES * S::Q_BYTES);
 #pragma unroll
-        for (int g = 0; g < 2; ++g)
+        for (int g = 0; g < TILES; ++g)
 #pragma unroll
           for (int c = 0; c < NCH; ++c)
             tma_load_2d(sQ + g * S::Q_BYTES + c * (FA_BM * 128), &tmQ, q_full, h * D + c * 64, q_off + q0 + g * FA_BM);
@@ -166,45 +168,70 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         constexpr uint32_t idesc_s = make_idesc(FA_BM, FA_BN, 1, 1, 0, 0);
         constexpr uint32_t idesc_o = make_idesc(FA_BM, D, 1, 1, 0, 1);  // A = P in TMEM, B = V read MN-major
         auto issue_s = [&](int g, int j) {
+          const int buf = TILES == 2 ? g : j & 1;
           const uint32_t q_addr = smem_u32(sQ + g * S::Q_BYTES), k_addr = smem_u32(sK + (j % FA_KV_STAGES) * S::KV_BYTES);
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
             const uint32_t off = (k >> 2) * (FA_BM * 128) + (k & 3) * 32;
-            umma_f16(tmem_base + g * FA_BN, make_smem_desc(q_addr + off, 16, 1024, UMMA_SWIZZLE_128B),
+            umma_f16(tmem_base + buf * FA_BN, make_smem_desc(q_addr + off, 16, 1024, UMMA_SWIZZLE_128B),
                      make_smem_desc(k_addr + off, 16, 1024, UMMA_SWIZZLE_128B), idesc_s, k != 0 ? 1u : 0u);
           }
-          umma_commit(&s_full[g]);
+          umma_commit(&s_full[buf]);
+        };
+        // P of the key tile in score buffer `buf` times V
+        auto issue_o = [&](int g, int buf, int j) {
+          const uint32_t v_addr = smem_u32(sV + (j % FA_KV_STAGES) * S::KV_BYTES);
+#pragma unroll
+          for (int k = 0; k < FA_BN / 16; ++k) {
+            // A: 16 keys = 8 TMEM columns; B = V tile [128 keys, D]: MN-major, 16 keys = 2048 B, 64-wide chunks of the head dim
+            // FA_BN * 128 B apart
+            umma_f16_ts(tmem_base + 2 * FA_BN + g * D, tmem_base + buf * FA_BN + k * 8,
+                        make_smem_desc(v_addr + k * 2048, FA_BN * 128, 1024, UMMA_SWIZZLE_128B), idesc_o, (j != 0 || k != 0) ? 1u : 0u);
+          }
         };
         bool ok = mbar_wait(q_full, 0, cta_abort, status, ERR_WAIT_FULL) &&
                   mbar_wait(&k_full[0], 0, cta_abort, status, ERR_WAIT_FULL);
         if (ok) {
           tc_fence_after();
-          for (int g = 0; g < 2; ++g)
+          for (int g = 0; g < TILES; ++g)
             if (n_of[g] > 0) issue_s(g, 0);
           umma_commit(&k_empty[0]);
         }
         for (int j = 0; j < n_kv && ok; ++j) {
+          auto next_scores = [&](int g) {
+            ok = mbar_wait(&k_full[(j + 1) % FA_KV_STAGES], ((j + 1) / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+            if (!ok) return;
+            tc_fence_after();
+            issue_s(g, j + 1);
+          };
+          if constexpr (TILES == 1) {
+            // the next scores go to the other buffer, whose P the product of tile j - 1 reads: products of one CTA run in the order they are
+            // issued in
+            if (j + 1 < n_kv) {
+              next_scores(0);
+              if (!ok) break;
+              umma_commit(&k_empty[(j + 1) % FA_KV_STAGES]);
+            }
+            ok = mbar_wait(&v_full[j % FA_KV_STAGES], (j / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL) &&
+                 mbar_wait(&p_full[0], j & 1, cta_abort, status, ERR_WAIT_TMEM_EMPTY);
+            if (!ok) break;
+            tc_fence_after();
+            issue_o(0, j & 1, j);
+            umma_commit(&v_empty[j % FA_KV_STAGES]);
+            umma_commit(&o_full[0]);
+            continue;
+          }
           ok = mbar_wait(&v_full[j % FA_KV_STAGES], (j / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
-          const uint32_t v_addr = smem_u32(sV + (j % FA_KV_STAGES) * S::KV_BYTES);
-          for (int g = 0; g < 2 && ok; ++g) {
+          for (int g = 0; g < TILES && ok; ++g) {
             if (j >= n_of[g]) continue;
             ok = mbar_wait(&p_full[g], j & 1, cta_abort, status, ERR_WAIT_TMEM_EMPTY);
             if (!ok) break;
             tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < FA_BN / 16; ++k) {
-              // A: 16 keys = 8 TMEM columns; B = V tile [128 keys, D]: MN-major, 16 keys = 2048 B, 64-wide chunks of the head dim
-              // FA_BN * 128 B apart
-              umma_f16_ts(tmem_base + 2 * FA_BN + g * D, tmem_base + g * FA_BN + k * 8,
-                          make_smem_desc(v_addr + k * 2048, FA_BN * 128, 1024, UMMA_SWIZZLE_128B), idesc_o, (j != 0 || k != 0) ? 1u : 0u);
-            }
+            issue_o(g, g, j);
             if (j + 1 == n_of[g]) umma_commit(&o_full[g]);
-            if (j + 1 < n_of[g]) {
-              // the next scores replace P: products of one CTA run in the order they are issued in
-              ok = mbar_wait(&k_full[(j + 1) % FA_KV_STAGES], ((j + 1) / FA_KV_STAGES) & 1, cta_abort, status, ERR_WAIT_FULL);
+            if (j + 1 < n_of[g]) {  // the next scores replace P: products run in order
+              next_scores(g);
               if (!ok) break;
-              tc_fence_after();
-              issue_s(g, j + 1);
             }
           }
           if (!ok) break;
@@ -214,10 +241,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     } else {
       // ------------------------------------------------------------------ softmax + epilogue
-      const int quarter = warp & 3, g = (warp - 2) >> 2;
+      const int quarter = warp & 3, g = TILES == 2 ? (warp - 2) >> 2 : 0;
       const int row = quarter * 32 + lane;  // query row inside the tile = TMEM lane
       const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      const uint32_t s_addr = lane_addr + g * FA_BN, o_addr = lane_addr + 2 * FA_BN + g * D;
+      const uint32_t o_addr = lane_addr + 2 * FA_BN + g * D;
       const float c_log2 = scale * 1.4426950408889634f;
       const uint64_t c2 = f2_pack(c_log2, c_log2);
       const int r0 = q0 + g * FA_BM;
@@ -227,7 +254,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       float m_run = -INFINITY, l_run = 0.f;
       bool ok = true;
       for (int j = 0; j < n_my; ++j) {
-        ok = mbar_wait(&s_full[g], j & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
+        const int buf = TILES == 2 ? g : j & 1;
+        const uint32_t s_addr = lane_addr + buf * FA_BN;
+        ok = mbar_wait(&s_full[buf], (TILES == 2 ? j : j >> 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -263,10 +292,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         row_max(2);
         const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * c_log2;  // scale > 0: the maximum commutes with the scaling
         const float m_new = fmaxf(m_run, mx);
+        bool seen = TILES == 2 || j == 0;  // one tile: every product's end is waited for, in turn (a phase that is left out could be mistaken)
         if (j == 0) {
           m_run = (m_new == -INFINITY) ? 0.f : m_new;
-        } else if (__any_sync(0xffffffffu, m_new > m_run + 8.f)) {
-          // the scores just read came after the product of the tile before: O may be corrected
+        } else if (__any_sync(0xffffffffu, qi < q_len && m_new > m_run + 8.f)) {  // (rows behind the segment have no say)
+          // O may be corrected once the product of the tile before is done; with two tiles it is, since the scores just read came after it
+          if constexpr (TILES == 1) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&o_full[0], (j - 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL));
+            if (!ok) break;
+            tc_fence_after();
+            seen = true;
+          }
           const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
           const float f = fa_exp2(m_run - m_use);  // <= 1
           l_run *= f;
@@ -303,6 +339,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
           tmem_st_32x16(s_addr + c4 * 16, pk);
         }
+        if (!seen) {  // (with the exponentials behind, this does not wait any more)
+          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[0], (j - 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL));
+          if (!ok) break;
+        }
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -313,7 +353,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // ---- epilogue: O / l -> bf16 -> staged through shared memory (the group's Q tile) -> coalesced rows of `out`
       if (ok && n_my > 0) {
-        ok = mbar_wait(&o_full[g], 0, cta_abort, status, ERR_WAIT_TMEM_FULL);
+        ok = mbar_wait(&o_full[g], TILES == 2 ? 0 : (n_my - 1) & 1, cta_abort, status, ERR_WAIT_TMEM_FULL);
         ok = __all_sync(0xffffffffu, ok);
       }
       if (ok && r0 < q_len) {
@@ -369,21 +409,42 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 1) tmem_dealloc(tmem_base, S::TMEM_COLS);
 }
 
-template <int D>
+template <int D, int TILES>
 static int launch_flash_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* seg, int nseg,
                             int max_q_tiles, int Tq, int Tk, int Hq, int Hkv, int q_stride, int k_stride, int v_stride,
                             int out_stride, int lse_stride, float scale, int* status, cudaStream_t s) {
-  using S = FaSmem<D>;
+  using S = FaSmem<D, TILES>;
   const CUtensorMap tq = make_tmap_2d(q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tq, size_t(Hq) * D, size_t(q_stride) * 2, FA_BM, 64,
                                       CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap tk = make_tmap_2d(k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, size_t(Hkv) * D, size_t(k_stride) * 2, FA_BN, 64,
                                       CU_TENSOR_MAP_SWIZZLE_128B);
   const CUtensorMap tv = make_tmap_2d(v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, Tk, size_t(Hkv) * D, size_t(v_stride) * 2, FA_BN, 64,
                                       CU_TENSOR_MAP_SWIZZLE_128B);
-  auto kern = flash_fwd_kernel<D>;
+  auto kern = flash_fwd_kernel<D, TILES>;
   if (cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), S::TOTAL); e != cudaSuccess) return (int)e;
-  return (int)launch_pdl(kern, dim3(static_cast<unsigned>(max_q_tiles) * Hq), dim3(FA_THREADS), S::TOTAL, s, tq, tk, tv,
+  return (int)launch_pdl(kern, dim3(static_cast<unsigned>(max_q_tiles) * Hq), dim3(S::THREADS), S::TOTAL, s, tq, tk, tv,
                          reinterpret_cast<__nv_bfloat16*>(out), lse, seg, nseg, Hq, Hkv, max_q_tiles, out_stride, lse_stride, scale, status);
+}
+
+// One tile a CTA where the CTAs of single tiles are no more than the SMs: two tiles a CTA would leave half of them idle, and a CTA of one tile
+// ends earlier (two tiles -> one, us: 397 rows, 14 heads of 64 12.5 -> 9.6, 32 heads of 128 14.3 -> 10.7; 300
+// rows behind 3000 59 -> 40; 1000 rows behind 8000, 14 heads of 64, 112 CTAs 138 -> 92). A row's
+// arithmetic is the same in both, and so are its bits.
+static int launch_flash_fwd_tiles(int D, const void* q, const void* k, const void* v, void* out, float* lse, const int* seg, int nseg,
+                                  int max_q_tiles, int Tq, int Tk, int Hq, int Hkv, int q_stride, int k_stride, int v_stride,
+                                  int out_stride, int lse_stride, float scale, int* status, cudaStream_t s) {
+  int dev = 0, sms = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return (int)e;
+  if (cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); e != cudaSuccess) return (int)e;
+  const int held = nseg < Tq ? nseg : Tq;  // segments that can have rows
+  const int singles = (Tq - held) / FA_BM + held;  // tiles there can be at most
+  const bool one = static_cast<long>(singles) * Hq <= sms;
+  auto run = [&](auto launch) {
+    return launch(q, k, v, out, lse, seg, nseg, one ? singles : max_q_tiles, Tq, Tk, Hq, Hkv, q_stride, k_stride, v_stride, out_stride,
+                  lse_stride, scale, status, s);
+  };
+  if (D == 64) return one ? run(launch_flash_fwd<64, 1>) : run(launch_flash_fwd<64, 2>);
+  return one ? run(launch_flash_fwd<128, 1>) : run(launch_flash_fwd<128, 2>);
 }
 
 }  // namespace sb
@@ -399,12 +460,9 @@ extern "C" int sb_flash_fwd(const void* q, const void* k, const void* v, void* o
   if (nseg <= 0 || max_q_tiles <= 0 || Tq <= 0) return 0;
   if (Hkv <= 0 || Hq % Hkv != 0) return (int)cudaErrorInvalidValue;
   try {
-    if (D == 64)
-      return sb::launch_flash_fwd<64>(q, k, v, out, lse, seg, nseg, max_q_tiles, Tq, Tk, Hq, Hkv, q_stride, k_stride, v_stride,
-                                      out_stride, lse_stride, scale, status, s);
-    if (D == 128)
-      return sb::launch_flash_fwd<128>(q, k, v, out, lse, seg, nseg, max_q_tiles, Tq, Tk, Hq, Hkv, q_stride, k_stride,
-                                       v_stride, out_stride, lse_stride, scale, status, s);
+    if (D == 64 || D == 128)
+      return sb::launch_flash_fwd_tiles(D, q, k, v, out, lse, seg, nseg, max_q_tiles, Tq, Tk, Hq, Hkv, q_stride, k_stride, v_stride, out_stride,
+                                        lse_stride, scale, status, s);
   } catch (const std::exception& e) {
     sb::set_last_error(e.what());
     return (int)cudaErrorInvalidValue;

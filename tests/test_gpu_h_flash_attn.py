@@ -213,3 +213,24 @@ def test_flash_backward_in_any_number_of_parts(kernels, monkeypatch, parts, lens
     for a, b in zip(got[0][1:], got[1][1:]):
         assert (b[-3:] == 5).all()
         torch.testing.assert_close(a, b, rtol=2**-7, atol=2.0**-16 * float(a[:-3].abs().max()))
+
+
+@pytest.mark.parametrize("Hq,Hkv,D", [(14, 2, 64), (8, 2, 128), (2, 1, 128)])
+@pytest.mark.parametrize("q_len,k_len", [(1, 1), (1, 700), (128, 128), (129, 129), (300, 301), (397, 397), (640, 640), (260, 2000)])
+def test_flash_forward_one_tile_per_cta(kernels, Hq, Hkv, D, q_len, k_len):
+    """Few tiles have a CTA each, many go in pairs: a segment's rows have the same bits alone (one tile a CTA) and in front of enough others
+    (pairs). Large scores make the running maximum rise."""
+    from slime_b200.ops import _lib, attention
+
+    torch.manual_seed(q_len + k_len)
+    more = 148 // Hq * 128 + 256  # rows: more tiles than SMs
+    q = (torch.randn(q_len + more, Hq, D, device="cuda") * 4).to(torch.bfloat16)
+    k, v = (torch.randn(k_len + more, Hkv, D, device="cuda").to(torch.bfloat16) for _ in range(2))
+    one = torch.tensor([[0, q_len, 0, k_len]], dtype=torch.int32, device="cuda")
+    both = torch.cat([one, torch.tensor([[q_len, more, k_len, more]], dtype=torch.int32, device="cuda")])
+    alone, lse = attention.flash_fwd(q[:q_len], k[:k_len], v[:k_len], one, D**-0.5)
+    among, lse_among = attention.flash_fwd(q, k, v, both, D**-0.5)
+    _lib.check_status("cuda")
+    assert torch.equal(alone, among[:q_len]) and torch.equal(lse, lse_among[:, :q_len])
+    want = _ref(q[:q_len], k[:k_len], v[:k_len], one.cpu(), D**-0.5)
+    assert float((alone.float() - want).norm() / want.norm()) < 2 * 2**-8
