@@ -82,6 +82,8 @@ def flash_fwd(q, k, v, seg, scale, max_q_len_hint: int | None = None, out=None, 
     Tq, Hq, D = q.shape
     Tk, Hkv = k.shape[0], k.shape[1]
     assert D in (64, 128), f"flash attention kernels cover head dims 64 and 128, not {D}"
+    if scale <= 0:  # the kernel hides scores as -infinity before it scales them: the sign goes to q, and 0 becomes a factor that rounds away
+        q, scale = (-q, -scale) if scale < 0 else (q, 1e-30)
     q, k, v = (t if _strides_ok(t) else t.contiguous() for t in (q, k, v))
     if out is None:
         out = (torch.zeros if zero_uncovered else torch.empty)(Tq, Hq, D, dtype=q.dtype, device=q.device)

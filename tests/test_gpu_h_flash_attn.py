@@ -234,3 +234,24 @@ def test_flash_forward_one_tile_per_cta(kernels, Hq, Hkv, D, q_len, k_len):
     assert torch.equal(alone, among[:q_len]) and torch.equal(lse, lse_among[:, :q_len])
     want = _ref(q[:q_len], k[:k_len], v[:k_len], one.cpu(), D**-0.5)
     assert float((alone.float() - want).norm() / want.norm()) < 2 * 2**-8
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+@pytest.mark.parametrize("lens", [[129], [300, 40, 1], [500] * 40])
+def test_flash_attention_takes_any_factor(kernels, scale, lens):
+    """Zero (the mean of the visible values) and negative factors, masked tiles included, with their gradients."""
+    from slime_b200.ops import _lib, attention
+
+    torch.manual_seed(len(lens))
+    seg = attention.segments_from_cu_seqlens(torch.tensor([0] + lens, device="cuda").cumsum(0))
+    ins = [torch.randn(sum(lens), h, 64, device="cuda").bfloat16() for h in (4, 2, 2)]
+    g = torch.randn(sum(lens), 4, 64, device="cuda").bfloat16()
+    res = []
+    for fn, cast in ((attention.segment_attention, lambda t: t), (lambda *a: _ref(*a[:3], a[3].cpu(), a[4]), lambda t: t.float())):
+        xs = [cast(t).clone().requires_grad_() for t in ins]
+        y = fn(*xs, seg, scale)
+        y.backward(g.to(y.dtype))
+        res.append([y.detach().float()] + [x.grad.float() for x in xs])
+    _lib.check_status("cuda")
+    for a, b in zip(*res):
+        assert float((a - b).norm()) <= 3 * 2**-8 * float(b.norm())
