@@ -4,6 +4,8 @@
 //   * vocab(-parallel) softmax statistics over fp32 logits rows: max, sum-exp, target logit,
 //     sum p*z  ->  log-prob and entropy; and the matching dlogits kernel
 //   * GRPO / PPO-clip / CISPO per-token surrogate with its derivative wrt log-prob
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace sb {
@@ -194,12 +196,14 @@ dlogits_kernel(const float* __restrict__ logits, const int* __restrict__ targets
 // mode 0: PPO/GRPO clip (optional dual clip eps_c > 1), mode 1: CISPO.
 // Inputs per token: logp (new), old_logp, adv, w (loss weight: mask / normaliser).
 // Outputs: g_lp[t] = d(sum_t w_t L_t)/d logp_t, and acc[0..3] += {sum w L, sum w clipfrac, sum w (old-new), sum w}
+// The CTAs of a cluster (or one alone) add their sums up in a fixed order. Bound by the latency of a thread's loads and of the reductions, us,
+// one CTA -> eight: 1000 rows 3.3 -> 4.1, 4096 rows 4.5 -> 4.3, 16384 rows 8.6 -> 4.5.
 __global__ void __launch_bounds__(1024)
 pg_loss_kernel(const float* __restrict__ logp, const float* __restrict__ old_logp, const float* __restrict__ adv,
                const float* __restrict__ w, const float* __restrict__ tis, float* __restrict__ g_lp,
                float* __restrict__ per_token_loss, float* __restrict__ acc, int T, float eps_lo, float eps_hi, float eps_c,
                int mode) {
-  // sums of thousands of terms of either sign: in 64 bits, rounded once a block
+  // sums of thousands of terms of either sign: in 64 bits, rounded once a cluster
   __shared__ double scratch[4][32];
   double sums[4] = {0., 0., 0., 0.};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
@@ -241,11 +245,22 @@ pg_loss_kernel(const float* __restrict__ logp, const float* __restrict__ old_log
     if (lane == 0) scratch[i][warp] = sums[i];
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  __shared__ double block_sum[4];
+  if (warp < 4) {
+    double v = lane < warps ? scratch[warp][lane] : 0.;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) block_sum[warp] = v;
+  }
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const bool many = cluster.num_blocks() > 1;
+  if (many) cluster.sync();
+  else __syncthreads();
+  if (cluster.block_rank() == 0 && threadIdx.x < 4) {
     double v = 0.;
-    for (int i = 0; i < warps; ++i) v += scratch[threadIdx.x][i];
+    for (unsigned r = 0; r < cluster.num_blocks(); ++r) v += cluster.map_shared_rank(block_sum, r)[threadIdx.x];
     atomicAdd(acc + threadIdx.x, static_cast<float>(v));
   }
+  if (many) cluster.sync();  // no CTA leaves while its sums may be read
 }
 
 }  // namespace sb
@@ -305,9 +320,21 @@ extern "C" int sb_pg_loss(const float* logp, const float* old_logp, const float*
                           float* g_lp, float* per_token_loss, float* acc, int T, float eps_lo, float eps_hi, float eps_c,
                           int mode, cudaStream_t s) {
   if (T == 0) return 0;
-  // one block adds a chunk's sums in a fixed order; more rows than a chunk has go to as many blocks as fill the SMs
-  const int blocks = T <= 16384 ? 1 : 148;
-  sb::pg_loss_kernel<<<blocks, 1024, 0, s>>>(logp, old_logp, adv, w, tis, g_lp, per_token_loss, acc, T, eps_lo, eps_hi,
-                                           eps_c, mode);
-  return (int)cudaGetLastError();
+  // a chunk's sums are added up in a fixed order, by one CTA or, where that takes longer than a cluster to meet, by eight; more rows than a
+  // chunk has go to as many CTAs as there are SMs
+  if (T <= 2048 || T > 16384) {
+    sb::pg_loss_kernel<<<T <= 2048 ? 1 : 148, 1024, 0, s>>>(logp, old_logp, adv, w, tis, g_lp, per_token_loss, acc, T, eps_lo, eps_hi, eps_c, mode);
+    return (int)cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(8);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 8;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, sb::pg_loss_kernel, logp, old_logp, adv, w, tis, g_lp, per_token_loss, acc, T, eps_lo, eps_hi, eps_c, mode);
 }

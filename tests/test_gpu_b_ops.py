@@ -403,3 +403,24 @@ def test_norms_refuse_weights_off_a_16_byte_boundary(kernels):
         ops.rmsnorm(x, w)
     y, _ = ops.rmsnorm(x.requires_grad_(), torch.ones(64, device="cuda", dtype=torch.bfloat16))
     assert torch.isfinite(y).all()
+
+
+@pytest.mark.parametrize("T", [1, 1025, 2048, 2049, 5000, 16384, 16385, 70001])
+def test_policy_loss_sums_of_any_length(kernels, T):
+    """One CTA, a cluster of eight, a CTA per SM: every token's gradient is written once, and the sums are those of 64 bits, rounded once a
+    cluster or CTA and once more as it is added (2^-24 each, 148 at most); up to a chunk they are the same on every run."""
+    from slime_b200.ops import _lib
+
+    torch.manual_seed(T)
+    lp, old, adv = (torch.randn(T, device="cuda") * s for s in (0.1, 0.1, 1.0))
+    w = torch.rand(T, device="cuda")
+    runs = []
+    for _ in range(3):
+        g, each, acc = torch.full((T,), float("nan"), device="cuda"), torch.empty(T, device="cuda"), torch.zeros(4, device="cuda")
+        args = [t.data_ptr() for t in (lp, old, adv, w)]
+        _lib.check(_lib.lib().sb_pg_loss(*args, None, g.data_ptr(), each.data_ptr(), acc.data_ptr(), T, 0.2, 0.28, 0.0, 0, _lib.stream()), "sb_pg_loss")
+        runs.append((g, acc))
+    assert torch.isfinite(g).all() and (T > 16384 or all(torch.equal(a, b) for r in runs for a, b in zip(r, runs[0])))
+    kl = (old - lp).double()
+    for got, terms in ((acc[0], each.double() * w), (acc[2], kl * w), (acc[3], w.double())):
+        assert abs(float(got) - float(terms.sum())) <= 2 * (148 if T > 16384 else 1) * 2.0**-24 * float(terms.abs().sum())
