@@ -69,13 +69,13 @@ group_fp8_quant_1x128_kernel(const __nv_bfloat16* __restrict__ x, __nv_fp8_e4m3*
   }
 }
 
-// The same for rows of whole 16-byte pieces: 16 lanes per group, 8 elements each, four groups' loads in flight. Bound by HBM; with one
+// The same for rows of whole 16-byte pieces: 16 lanes per group, 8 elements each, AHEAD groups' loads in flight. Bound by HBM; with one
 // 8-byte load a lane in flight and 64-bit divisions 3465 x 9728 took 49 us; all four widths of a Qwen3-4B layer
 // 111 -> 65 us.
+template <int AHEAD>
 __global__ void __launch_bounds__(256)
 group_fp8_quant_1x128_vec_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale_inv,
                                  float* __restrict__ scale_t, int M, uint32_t groups, size_t ldx, size_t ldq, int pow2_scale) {
-  constexpr int AHEAD = 4;
   pdl_wait();
   pdl_launch_dependents();
   const int sub = threadIdx.x & 15;
@@ -128,9 +128,13 @@ static cudaError_t launch_group_quant(const void* x, void* q, float* scale_inv, 
   const long total = (long)M * groups;
   if (ldx % 8 == 0 && ldq % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0 &&
       total < (1l << 30)) {
-    const long blocks = (total + 63) / 64;  // 16 groups a block at a time, four deep
-    return launch_pdl(group_fp8_quant_1x128_vec_kernel, dim3(static_cast<unsigned>(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, s,
-                      (const __nv_bfloat16*)x, (uint8_t*)q, scale_inv, scale_t, M, static_cast<uint32_t>(groups), (size_t)ldx, (size_t)ldq, pow2_scale);
+    // 16 groups a block at a time; four deep only where a group for every 16 lanes fills the SMs (8 x 2560: 2.9 us four deep, 1.8 one deep;
+    // 4000 x 9728: 32 four deep)
+    const bool deep = total > 148l * 8 * 16;
+    const long blocks = deep ? (total + 63) / 64 : (total + 15) / 16;
+    return launch_pdl(deep ? group_fp8_quant_1x128_vec_kernel<4> : group_fp8_quant_1x128_vec_kernel<1>,
+                      dim3(static_cast<unsigned>(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, s, (const __nv_bfloat16*)x, (uint8_t*)q, scale_inv,
+                      scale_t, M, static_cast<uint32_t>(groups), (size_t)ldx, (size_t)ldq, pow2_scale);
   }
   const long blocks = (total + 7) / 8;
   group_fp8_quant_1x128_kernel<<<static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(

@@ -137,7 +137,7 @@ def test_fp8_engine_on_gpu_tracks_the_bf16_engine(kernels):
         e.shutdown()
 
 
-@pytest.mark.parametrize("M,K", [(1, 128), (3, 384), (777, 9728), (4000, 128)])
+@pytest.mark.parametrize("M,K", [(1, 128), (3, 384), (777, 9728), (4000, 128), (148, 16384), (149, 16384)])
 @pytest.mark.parametrize("pow2", [0, 1])
 def test_activation_quant_in_16_byte_pieces(kernels, M, K, pow2):
     """Rows of whole 16-byte pieces and rows that are not take different kernels: the same bits, also for zeros, infinities and NaN."""
