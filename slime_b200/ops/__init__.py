@@ -394,7 +394,7 @@ class _RMSNorm(torch.autograd.Function):
             part = torch.empty(n, H, dtype=torch.float32, device=dy.device)
             held = getattr(weight, "main_grad", None)
             direct = held is not None and held.dtype == torch.float32 and held.is_contiguous() and T > 0
-            dw = held if direct else torch.empty(H, dtype=torch.float32, device=dy.device)
+            dw = held if direct else (torch.empty if T else torch.zeros)(H, dtype=torch.float32, device=dy.device)  # no rows: no launch
             rc = _lib.lib().sb_rmsnorm_bwd(P(dy2), P(h), P(weight), P(rstd), P(dres), P(dh), P(part), P(dw), T, H, n, int(direct),
                                            _lib.stream())
             _lib.check(rc, "sb_rmsnorm_bwd")
@@ -499,7 +499,7 @@ def _head_norm_bwd(x, dy, w, eps):
         dh = torch.empty_like(x2)
         n = min(_norm_ctas(x.device), max(rows, 1))
         part = torch.empty(n, D, dtype=torch.float32, device=x.device)
-        dw = torch.empty(D, dtype=torch.float32, device=x.device)
+        dw = (torch.empty if rows else torch.zeros)(D, dtype=torch.float32, device=x.device)  # no rows: no launch
         rc = _lib.lib().sb_rmsnorm_bwd(P(dy2), P(x2), P(w), P(rstd), None, P(dh), P(part), P(dw), rows, D, n, 0,
                                        _lib.stream())
         _lib.check(rc, "sb_rmsnorm_bwd(head)")

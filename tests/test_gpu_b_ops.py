@@ -424,3 +424,23 @@ def test_policy_loss_sums_of_any_length(kernels, T):
     kl = (old - lp).double()
     for got, terms in ((acc[0], each.double() * w), (acc[2], kl * w), (acc[3], w.double())):
         assert abs(float(got) - float(terms.sum())) <= 2 * (148 if T > 16384 else 1) * 2.0**-24 * float(terms.abs().sum())
+
+
+def test_norms_over_no_rows_gain_no_gradient(kernels):
+    """Layer norm and per-head norm, with ``main_grad`` and without."""
+    from slime_b200 import ops
+
+    for held in (True, False):
+        w, hw = (torch.ones(n, device="cuda", dtype=torch.bfloat16).requires_grad_() for n in (128, 64))
+        for t in (w, hw):
+            if held:
+                t.main_grad = torch.ones(t.numel(), device="cuda")
+        x = torch.empty(0, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+        y, h = ops.rmsnorm(x, w)
+        junk = [torch.full((n,), 7.0, device="cuda") for n in (64, 64, 128, 128, 256)]
+        del junk  # what new buffers are made of
+        torch.autograd.backward([y, h], [torch.empty_like(y), torch.empty_like(h)])
+        heads = torch.empty(0, 2, 64, device="cuda", dtype=torch.bfloat16)
+        _, dhw = ops._head_norm_bwd(heads, heads, hw, 1e-6)
+        for t, g in ((w, w.grad), (hw, dhw)):
+            assert (t.main_grad == 1).all() and g is None if held else (g == 0).all()
