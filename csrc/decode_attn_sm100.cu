@@ -191,9 +191,10 @@ decode_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 
   // warp 0, all lanes: start the copies of the K (or V) half of tile i. Lane p fetches the block-table entry of page p
   // and issues that page's boxes (one per 64-wide chunk of the head dim), so the table reads overlap. K and V have
-  // separate barriers because their buffers become free at different times: K once S^T of the tile two back is done,
-  // V once that tile's O^T is done. With three stages K runs three tiles ahead of the softmax and V two.
-  // buffer, barrier and phase of the K (or V) half of tile i
+  // separate barriers because their buffers become free at different times. Three stages: K's once S^T of the tile three back is done, V's
+  // once that tile's O^T is, so that K runs three tiles ahead of the softmax and V two. Three halves: half n (K of tile n / 2, or its V)
+  // takes the slot of half n - 3, a V behind O^T or a K behind S^T, so that one tile is in flight beside the one that is worked on.
+  // Buffer, barrier and phase of the K (or V) half of tile i:
   auto half_buf = [&](int i, bool is_k) -> uint8_t* {
     if constexpr (S::HALVES) return sKV + (2 * i + (is_k ? 0 : 1)) % 3 * S::KV_TILE;
     return sKV + i % DA_STAGES * S::STAGE + (is_k ? S::KV_TILE : 0);

@@ -8,7 +8,7 @@
 namespace sb {
 
 constexpr int NORM_THREADS = 256;
-constexpr int NORM_MAX_VEC = 4;  // up to 4 x 8 bf16 per thread cached in registers -> H <= 8192
+constexpr int NORM_MAX_H = 8192;  // widest row of a block: 1024 threads with a vector of 8 each
 
 struct bf16x8 {
   uint4 u;
@@ -359,13 +359,14 @@ static cudaError_t launch_rmsnorm_bwd(const __nv_bfloat16* dy, const __nv_bfloat
 // ---------------------------------------------------------------- QK-norm + RoPE
 // x: [T, heads_total, D] packed (q heads then k heads then v heads in one qkv row is fine:
 // `row_stride` is the element pitch of a token, `head0` the first head to process, `nheads`
-// how many). One warp per (token, head). Rotate-half convention:
+// how many). Rotate-half convention:
 //   o[i] = a[i] cos - a[i+D/2] sin ; o[i+D/2] = a[i+D/2] cos + a[i] sin
 // with a = x or rmsnorm_D(x) * nw when nw != nullptr. cos/sin table: [max_pos, D/2] fp32.
 // `sign` = +1 forward rotation, -1 inverse rotation (backward of RoPE).
 // A group of D / 16 lanes has a head: each lane eight neighbouring elements of its lower half and the eight they are turned with, as
 // 16-byte accesses. Bound by HBM; with a warp per head and 2-byte accesses the instructions bound it (15800 tokens, 14 heads of 64:
-// 50 -> 8 us). VEC = false is that form, for rows that are no whole 16-byte pieces.
+// 50 -> 8 us). VEC = false is that form, a warp per (token, head), for rows that are no whole 16-byte
+// pieces.
 template <int D>
 __device__ __forceinline__ float head_sum(float v) {  // over the lanes of a head
 #pragma unroll
@@ -545,8 +546,8 @@ rope_norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
   }
 }
 
-// Inference form of the above, fused with the KV-cache write: one launch per layer instead of four. One warp per
-// (token, head) of a packed qkv row [T, (Hq + 2 Hkv) * D]:
+// Inference form of the above, fused with the KV-cache write: one launch per layer instead of four. Heads of a
+// packed qkv row [T, (Hq + 2 Hkv) * D], D / 16 lanes each (a warp each where VEC = false; a warp of the other form has heads of all three kinds):
 //   q heads  (per-head RMSNorm +) RoPE in place
 //   k heads  the same, written in place (prefill attends over the row itself) and to k_cache[slot[t], head]
 //   v heads  copied to v_cache[slot[t], head]
@@ -742,7 +743,7 @@ static inline bool norm_aligned(const void* a, const void* b, const void* c, con
 extern "C" int sb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                               int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_MAX_H || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_fwd((const bf16*)x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
@@ -750,7 +751,7 @@ extern "C" int sb_rmsnorm_fwd(const void* x, const void* res, const void* w, voi
 extern "C" int sb_rmsnorm_fwd_f32x(const float* x, const void* res, const void* w, void* y, void* res_out, float* rstd,
                                    int T, int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_MAX_H || !norm_aligned(x, res, w, y, res_out)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_fwd(x, (const bf16*)res, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, T, H, eps, s);
 }
 
@@ -759,7 +760,7 @@ extern "C" int sb_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
                               void* dh, float* dw_partial, float* dw, int T, int H, int num_ctas, int accumulate_dw,
                               cudaStream_t s) {
   if (T == 0) return 0;
-  if (H % 8 != 0 || H > sb::NORM_THREADS * sb::NORM_MAX_VEC * 8 || !norm_aligned(dy, h, w, dres_in, dh)) return (int)cudaErrorInvalidValue;
+  if (H % 8 != 0 || H > sb::NORM_MAX_H || !norm_aligned(dy, h, w, dres_in, dh)) return (int)cudaErrorInvalidValue;
   return (int)sb::launch_rmsnorm_bwd((const bf16*)dy, (const bf16*)h, (const bf16*)w, rstd, (const bf16*)dres_in,
                                      (bf16*)dh, dw_partial, dw, T, H, num_ctas, accumulate_dw, s);
 }
@@ -879,7 +880,7 @@ extern "C" int sb_add_bf16(const void* a, const void* b, void* out, long n, cuda
 
 #include "rmsnorm_bwd_static.h"
 
-static_assert(SB_RMSNORM_STATIC_MAX_H == sb::NORM_THREADS * sb::NORM_MAX_VEC * 8,
+static_assert(SB_RMSNORM_STATIC_MAX_H == sb::NORM_MAX_H,
               "the static scratch is sized for the widest row the norm kernels accept");
 
 // [SB_RMSNORM_STATIC_MAX_CTAS, SB_RMSNORM_STATIC_MAX_H] fp32, 4.6 MiB. In host code this name is only a host-side

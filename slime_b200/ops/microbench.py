@@ -76,7 +76,7 @@ def bench_gemm(a):
         x = torch.randn(M, K, device="cuda", dtype=bf)
         w = torch.randn(N, K, device="cuda", dtype=bf)
         fl = 2.0 * M * N * K
-        for bn in (128, 256):
+        for bn in (None, 128, 256):  # the plan that a call gets; the one-SM kernel in both widths
             t = time_ms(lambda: ops.gemm(x, w, bn=bn), a.iters)
             _emit(kind="nt", M=M, N=N, K=K, bn=bn, ms=t, tflops=fl / t / 1e9)
         if not a.no_cublas:
